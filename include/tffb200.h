@@ -182,7 +182,7 @@ int tff_nonbonded_atom_pairs(int dtype, int64_t natoms, const void *coords, int6
  * buffers, or a time-critical loop that must never reach an allocator (an allocation can
  * synchronise the device or fail mid-run). This entry point calls no cudaMalloc/cudaFree
  * and no allocating library routine; its scratch is a static device array inside
- * libtffb200 (about 3 MiB, held by every GPU that loads the library until exit), so natoms
+ * libtffb200 (about 6 MiB, held by every GPU that loads the library until exit), so natoms
  * is limited to TFF_NOALLOC_MAX_ATOMS (larger inputs return TFF_ERR_INVALID). The first
  * call on each device (and the first after a device reset) looks the array up with
  * cudaGetSymbolAddress: make it before any stream capture. All calls share the array
