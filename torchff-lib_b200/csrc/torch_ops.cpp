@@ -133,7 +133,7 @@ at::Tensor nblist_into(bool cell_list, const at::Tensor &coords, const OptT &box
   const OptT b = opt_ptr(box) ? OptT(cont(*box, x.scalar_type())) : std::nullopt;
   const OptT r = as_long(rp), c = as_long(col);
   const int64_t n = x.size(0);
-  at::Tensor npairs = at::zeros({1}, x.options().dtype(at::kInt));
+  at::Tensor npairs = at::empty({1}, x.options().dtype(at::kInt));
   if (!cell_list) {
     check(tff_nblist_nsquared(dt, n, ptr(x), ptr(b), cutoff, typed<const int64_t>(r), typed<const int64_t>(c),
                               include_self ? 1 : 0, typed<int64_t>(pairs), pairs.size(0), typed<int32_t>(npairs),
