@@ -273,7 +273,7 @@ int system_grad_impl(tff_system sys, const T *x, const T *box, const T *dir, dou
     } else {
       char *pw2 = static_cast<char *>(sys->pme_ws2);
       TFF_CUDA(cudaMemsetAsync(pw2 + sys->pl.zero_off, 0, sys->pl.zero_bytes, ps));
-      pme_spread_dir_kernel<T><<<nb, kPmeBlock, 0, ps>>>(atoms, dir, n, box, K,
+      pme_spread_dir_kernel<T><<<pme_blocks(n), kPmeBlock, 0, ps>>>(atoms, dir, n, box, K,
                                                          reinterpret_cast<S *>(pw2 + sys->pl.fix));
       TFF_LAUNCHED();
       T *psi_grid = nullptr;

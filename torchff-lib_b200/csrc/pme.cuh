@@ -24,39 +24,6 @@ namespace tff {
 
 constexpr int kPmeBlock = 256;
 
-// Per-atom stencil: origin index (already wrapped into [0,K)) and the 3x6 weights.
-template <class T>
-struct Stencil {
-  int g0[3];
-  T val[3][6];
-  T der[3][6];
-};
-
-// recip[d*3 + c] = K * inv[c][d]: u_d = sum_c recip[d][c] r_c
-template <class T>
-__device__ __forceinline__ void make_stencil(double rx, double ry, double rz, const double *recip, int K,
-                                             Stencil<T> &s) {
-  const double r[3] = {rx, ry, rz};
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double u = recip[3 * d] * r[0] + recip[3 * d + 1] * r[1] + recip[3 * d + 2] * r[2];
-    const double m0 = ceil(u);
-    const T w = (T)(m0 - u);
-    bspline6<T>(w, s.val[d], s.der[d]);
-    // first stencil point modulo K: one compare for atoms within a box length of the
-    // primary cell (the common case), a 64-bit remainder otherwise
-    long long g = (long long)m0 - 3;
-    if (g >= -K && g < 2 * (long long)K) {
-      g += g < 0 ? K : 0;
-      g -= g >= K ? K : 0;
-    } else {
-      g %= K;
-      if (g < 0) g += K;
-    }
-    s.g0[d] = (int)g;
-  }
-}
-
 struct PmeShared {
   double recip[9];
   double inv[9];
@@ -121,219 +88,134 @@ struct IndexedAtoms {
   }
 };
 
-// Spread: a group of kLanesPerAtom lanes per atom; lane g of the group takes the stencil
-// rows r = g, g + kLanesPerAtom, ... of the 36 (x, y) rows, 6 z points each. Loops run at
-// warp granularity so that every lane of a warp takes the same trip count. `bid` and
-// `nblk` are the block index and count over which the atoms are distributed.
-constexpr int kLanesPerAtom = 8;
-constexpr int kAtomsPerWarp = kWarp / kLanesPerAtom;
+// Stencils are computed by a warp for up to kStencilAtoms atoms at a time, one (atom, axis) per
+// lane, into shared memory: the lanes that work on an atom then read its weights instead of
+// evaluating the same splines each.
+constexpr int kStencilAtoms = 10;
 
-template <class T, class Atoms>
-__device__ __forceinline__ void spread_atoms(const Atoms &atoms, int64_t nthreads, const PmeShared &sh, int K,
-                                             typename Acc<T>::S *grid, int64_t bid, int64_t nblk) {
-  const int g = threadIdx.x % kLanesPerAtom;
-  const int64_t wglob = (bid * blockDim.x + threadIdx.x) / kWarp;
-  const int64_t nwarps = nblk * blockDim.x / kWarp;
-  for (int64_t wb = wglob * kAtomsPerWarp; wb < nthreads; wb += nwarps * kAtomsPerWarp) {
-    const int64_t t = wb + (threadIdx.x % kWarp) / kLanesPerAtom;
-    double rx, ry, rz;
-    T q;
-    if (t >= nthreads || !atoms.get(t, rx, ry, rz, q)) continue;
-    Stencil<T> s;
-    make_stencil<T>(rx, ry, rz, sh.recip, K, s);
-    for (int r = g; r < 36; r += kLanesPerAtom) {
-      const int a = r / 6, b = r % 6;
-      int gx = s.g0[0] + a, gy = s.g0[1] + b;
-      gx -= (gx >= K) ? K : 0;
-      gy -= (gy >= K) ? K : 0;
-      const T wxy = q * s.val[0][a] * s.val[1][b];
-      const int64_t row = ((int64_t)gx * K + gy) * K;
-      int gz = s.g0[2];
-#pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        Acc<T>::add(&grid[row + gz], (double)(wxy * s.val[2][c]));
-        gz = (gz + 1 == K) ? 0 : gz + 1;
-      }
-    }
+// One stencil point of an axis: weight and element offset of its index in the K^3 grid (the
+// index, wrapped into [0, K), times the axis's stride). Entries are vector-aligned for one load.
+template <class T> struct SplinePoint;
+template <> struct __align__(8) SplinePoint<float> { float w; int off; };
+template <> struct __align__(16) SplinePoint<double> { double w; int off; };
+
+// Weight and derivative.
+template <class T> struct SplinePoint2;
+template <> struct __align__(16) SplinePoint2<float> { float w, d; int off; };
+template <> struct __align__(16) SplinePoint2<double> { double w, d; int off; };
+
+template <class T>
+struct SpreadStage { SplinePoint<T> p[kStencilAtoms][3][6]; };
+template <class T>
+struct GatherStage { SplinePoint2<T> p[kStencilAtoms][3][6]; };
+
+// Spline argument and grid offsets of an atom on axis d: returns w (the weights are M6(w + k))
+// and calls put(k, offset) for the 6 points. recip[d*3 + c] = K * inv[c][d]: u_d = sum_c
+// recip[d][c] r_c. The first point is wrapped into [0, K) by compares for atoms within a box
+// length of the primary cell (the common case), by a 64-bit remainder otherwise.
+template <class F>
+__device__ __forceinline__ double axis_points(double rx, double ry, double rz, const PmeShared &sh, int K, int d,
+                                              F put) {
+  const double u = sh.recip[3 * d] * rx + sh.recip[3 * d + 1] * ry + sh.recip[3 * d + 2] * rz;
+  const double m0 = ceil(u);
+  long long g = (long long)m0 - 3;
+  if (g >= -K && g < 2 * (long long)K) {
+    g += g < 0 ? K : 0;
+    g -= g >= K ? K : 0;
+  } else {
+    g %= K;
+    if (g < 0) g += K;
   }
+  const int stride = d == 0 ? K * K : d == 1 ? K : 1;  // K <= 1024: offsets fit 32 bits
+  int at = (int)g;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    put(k, at * stride);
+    at = at + 1 == K ? 0 : at + 1;
+  }
+  return m0 - u;
 }
 
-// Spread in groups of kSpreadGroup consecutive atoms (FP32 inputs, fixed-point grid). The
-// atoms of a molecule are usually consecutive (a water's O, H, H), so their 6x6x6 stencils
-// overlap: a warp sums a group's contributions over the union window of its stencils (at
-// most kSpreadWin points per axis) and adds each window point to the grid with one atomic,
-// where the per-atom spread adds every contribution (3 x 216 for a water, against 7^3 = 343
-// window points for a typical one). Every contribution is rounded to fixed point by itself
-// and the integers are summed, exactly as the per-atom spread's atomics sum them, so the
-// grid is bit-identical to it. A group whose atoms lie too far apart on the grid (or whose
-// stencils are taken on a grid of fewer than kSpreadWin points) is spread atom by atom.
-constexpr int kSpreadGroup = 3;
-constexpr int kGroupsPerPass = 10;  // most groups staged per warp and pass: 30 atoms, one per lane
-constexpr int kSpreadWin = 8;
-
-struct GroupStencil {
-  int org[3];    // first stencil point per axis, ceil(u) - 3 wrapped into [0, K)
-  float w[3][6]; // B-spline weights
-  float q;
-  int valid;
-};
-
-// Grouped spread of atoms [0, n) by the blocks bid of nblk (warp-strided over groups); S is
-// the warp's stencil staging (kSpreadGroup * kGroupsPerPass entries in shared memory). Each
-// warp stages as many groups per pass as it takes for the groups to fill the warps.
-template <class Atoms>
-__device__ __forceinline__ void spread_groups(const Atoms &atoms, int64_t n, const PmeShared &sh, int K,
-                                              unsigned long long *grid, int64_t bid, int64_t nblk, GroupStencil *S) {
+// Spread of atoms [0, n) by the blocks bid of nblk. A warp takes its staged atoms one by one, six
+// lanes along z and five (x, y) rows at a time, so that an atomic instruction touches runs of six
+// consecutive grid points: 81 L2 sectors per atom, where lanes over the rows touched one for
+// each of the 216 points. FP32 contributions are rounded to fixed point one by one (the weight
+// of the x axis carries the charge and the scale, a power of two), so the grid does not depend
+// on the order of the atoms.
+//
+// Bound by the SM's reduction throughput (about one sector per clock) and L2 atomics. Alone: 300,000
+// atoms FP32 160 -> 126 us against groups of three atoms with a lane per row, 9,000 atoms 11.7 ->
+// 8.7 us; 30,000 scattered charges FP64 46 -> 20 us, 9,000 atoms 16.5 -> 9.5 us.
+template <class T, class Atoms>
+__device__ __forceinline__ void spread_atoms(const Atoms &atoms, int64_t n, const PmeShared &sh, int K,
+                                             typename Acc<T>::S *grid, int64_t bid, int64_t nblk,
+                                             SpreadStage<T> &S) {
   const int lane = threadIdx.x & 31;
   const int64_t wg = (bid * blockDim.x + threadIdx.x) / kWarp;
   const int64_t nw = nblk * blockDim.x / kWarp;
-  const int64_t groups = (n + kSpreadGroup - 1) / kSpreadGroup;
-  const int gpp = (int)min((int64_t)kGroupsPerPass, max((int64_t)1, (groups + nw - 1) / nw));
-  const int kAtoms = kSpreadGroup * gpp;
-  for (int64_t base = wg * kAtoms; base < n; base += nw * kAtoms) {
+  // as many atoms per pass as it takes for them to fill the warps
+  const int apw = (int)min((int64_t)kStencilAtoms, max((int64_t)1, (n + nw - 1) / nw));
+  const int r0 = lane / 6, c = lane - 6 * r0;
+  for (int64_t base = wg * apw; base < n; base += nw * apw) {
     __syncwarp();  // every lane is done with the previous pass's stencils
-    if (lane < kAtoms) {
-      GroupStencil &g = S[lane];
+    if (lane < 3 * apw) {
+      const int k = lane / 3, d = lane - 3 * k;
+      SplinePoint<T>(&p)[6] = S.p[k][d];
       double rx, ry, rz;
-      float qa;
-      const int64_t a = base + lane;
-      g.valid = a < n && atoms.get(a, rx, ry, rz, qa);
-      if (g.valid) {
-        const double r[3] = {rx, ry, rz};
-        float der[6];
+      T q;
+      if (base + k < n && atoms.get(base + k, rx, ry, rz, q)) {
+        const double w = axis_points(rx, ry, rz, sh, K, d, [&](int i, int off) { p[i].off = off; });
+        T val[6], der[6];
+        bspline6<T>((T)w, val, der);
+        if (d == 0) {
+          if (sizeof(T) == 4) q *= T(kFixScale);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double u = sh.recip[3 * d] * r[0] + sh.recip[3 * d + 1] * r[1] + sh.recip[3 * d + 2] * r[2];
-          const double m0 = ceil(u);
-          bspline6<float>((float)(m0 - u), g.w[d], der);
-          // first stencil point wrapped into [0, K) (the window code below relies on it):
-          // compares within a box length of the primary cell, a 64-bit remainder beyond
-          long long o = (long long)m0 - 3;
-          if (o >= -K && o < 2 * (long long)K) {
-            o += o < 0 ? K : 0;
-            o -= o >= K ? K : 0;
-          } else {
-            o %= K;
-            if (o < 0) o += K;
-          }
-          g.org[d] = (int)o;
+          for (int i = 0; i < 6; ++i) val[i] = q * val[i];
         }
-        g.q = qa;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) p[i].w = val[i];
+      } else {
+        p[0].off = -1;
       }
     }
     __syncwarp();
 #pragma unroll 1
-    for (int gi = 0; gi < gpp; ++gi) {
-      const GroupStencil *G = S + kSpreadGroup * gi;
-      // offsets of the atoms' stencils from the first valid atom's, taken modulo K into
-      // (-K/2, K/2], and the window's extent per axis
-      int first = -1;
+    for (int k = 0; k < apw; ++k) {
+      const auto &p = S.p[k];
+      if (p[0][0].off < 0 || lane >= 30) continue;
+      const SplinePoint<T> pz = p[2][c], py = p[1][r0];
+      const auto add = [&](const SplinePoint<T> &x, const SplinePoint<T> &y) {
+        const T v = (x.w * y.w) * pz.w;
+        const int at = x.off + y.off + pz.off;
+        if constexpr (sizeof(T) == 4)
+          atomicAdd(&grid[at], (unsigned long long)__float2ll_rn(v));
+        else
+          atomicAdd(&grid[at], v);
+      };
+      // rows (a, r0) for y indices 0..4, then the six rows of y index 5
 #pragma unroll
-      for (int k = kSpreadGroup - 1; k >= 0; --k)
-        if (G[k].valid) first = k;
-      if (first < 0) continue;
-      int rel[kSpreadGroup][3], lo[3], ext[3];
-      bool fits = K >= kSpreadWin;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        int mn = 0, mx = 0;
-#pragma unroll
-        for (int k = 0; k < kSpreadGroup; ++k) {
-          int v = G[k].org[d] - G[first].org[d];  // origins lie in [0, K) (wrapped above): |v| < K
-          if (v > K / 2) v -= K;
-          if (v <= -((K + 1) / 2)) v += K;
-          rel[k][d] = v;
-          if (G[k].valid) {
-            mn = min(mn, v);
-            mx = max(mx, v);
-          }
-        }
-        lo[d] = mn;
-        ext[d] = mx - mn + 6;
-        fits = fits && ext[d] <= kSpreadWin;
-      }
-      if (fits) {
-        // window point (x, y, z) in window coordinates; atom k covers it when
-        // 0 <= x - (rel_k - lo) < 6 on every axis
-        const int rows = ext[0] * ext[1];
-        for (int r = lane; r < rows; r += kWarp) {
-          const int ax = r / ext[1], ay = r % ext[1];
-          float wxy[kSpreadGroup];
-          int oz[kSpreadGroup];
-#pragma unroll
-          for (int k = 0; k < kSpreadGroup; ++k) {
-            const int ix = ax - (rel[k][0] - lo[0]), iy = ay - (rel[k][1] - lo[1]);
-            const bool in = G[k].valid && ix >= 0 && ix < 6 && iy >= 0 && iy < 6;
-            wxy[k] = in ? G[k].q * G[k].w[0][ix] * G[k].w[1][iy] : 0.f;
-            oz[k] = in ? rel[k][2] - lo[2] : 1 << 20;  // outside every z
-          }
-          // origin in [0, K), lo in (-K/2, 0], ax, ay < 8 <= K: one wrap either way
-          int gx = G[first].org[0] + lo[0] + ax, gy = G[first].org[1] + lo[1] + ay;
-          gx += gx < 0 ? K : 0;
-          gx -= gx >= K ? K : 0;
-          gy += gy < 0 ? K : 0;
-          gy -= gy >= K ? K : 0;
-          const int64_t row = ((int64_t)gx * K + gy) * K;
-          int gz = G[first].org[2] + lo[2];
-          gz += gz < 0 ? K : 0;
-          for (int z = 0; z < ext[2]; ++z) {
-            unsigned long long acc = 0ull;
-            bool any = false;
-#pragma unroll
-            for (int k = 0; k < kSpreadGroup; ++k) {
-              const int iz = z - oz[k];
-              if (iz >= 0 && iz < 6) {
-                acc += to_fix_f(wxy[k] * G[k].w[2][iz]);
-                any = true;
-              }
-            }
-            if (any) atomicAdd(&grid[row + gz], acc);
-            gz = (gz + 1 == K) ? 0 : gz + 1;
-          }
-        }
-      } else {
-        // atom by atom: lanes over the 36 (x, y) rows, 6 z points each
-#pragma unroll 1
-        for (int k = 0; k < kSpreadGroup; ++k) {
-          const GroupStencil &g = G[k];
-          if (!g.valid) continue;
-          for (int r = lane; r < 36; r += kWarp) {
-            const int a = r / 6, b = r % 6;
-            int gx = (g.org[0] + a) % K, gy = (g.org[1] + b) % K, gz = g.org[2] % K;
-            gx += gx < 0 ? K : 0;
-            gy += gy < 0 ? K : 0;
-            gz += gz < 0 ? K : 0;
-            const float wxy = g.q * g.w[0][a] * g.w[1][b];
-            const int64_t row = ((int64_t)gx * K + gy) * K;
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-              atomicAdd(&grid[row + gz], to_fix_f(wxy * g.w[2][c]));
-              gz = (gz + 1 == K) ? 0 : gz + 1;
-            }
-          }
-        }
-      }
+      for (int a = 0; a < 6; ++a) add(p[0][a], py);
+      const SplinePoint<T> p5 = p[1][5];
+      add(p[0][r0], p5);
+      if (r0 == 0) add(p[0][5], p5);
     }
   }
 }
 
-template <class Atoms>
-__global__ void __launch_bounds__(kPmeBlock) pme_spread_grouped_kernel(Atoms atoms, int64_t n, const float *box, int K,
-                                                                       unsigned long long *grid) {
-  __shared__ PmeShared sh;
-  __shared__ GroupStencil st[kPmeBlock / kWarp][kSpreadGroup * kGroupsPerPass];
-  if (threadIdx.x == 0) load_pme_shared(box, K, sh);
-  __syncthreads();
-  spread_groups(atoms, n, sh, K, grid, blockIdx.x, gridDim.x, st[threadIdx.x >> 5]);
-}
-
 template <class T, class Atoms>
-__global__ void __launch_bounds__(kPmeBlock) pme_spread_kernel(Atoms atoms, int64_t nthreads, const T *box, int K,
+__global__ void __launch_bounds__(kPmeBlock) pme_spread_kernel(Atoms atoms, int64_t n, const T *box, int K,
                                                                typename Acc<T>::S *grid) {
   __shared__ PmeShared sh;
+  __shared__ SpreadStage<T> st[kPmeBlock / kWarp];
   if (threadIdx.x == 0) load_pme_shared(box, K, sh);
   __syncthreads();
-  spread_atoms<T>(atoms, nthreads, sh, K, grid, blockIdx.x, gridDim.x);
+  spread_atoms<T>(atoms, n, sh, K, grid, blockIdx.x, gridDim.x, st[threadIdx.x >> 5]);
+}
+
+// Blocks of a kernel that takes one atom (spread) or kGatherAtomsPerWarp (gather) per warp at a
+// time, up to a few waves.
+inline int pme_blocks(int64_t warps) {
+  return (int)std::max<int64_t>(1, std::min<int64_t>((warps * kWarp + kPmeBlock - 1) / kPmeBlock, (int64_t)sm_count() * 8));
 }
 
 static __global__ void pme_fix_to_real_kernel(const unsigned long long *gi, float *gf, int64_t n) {
@@ -442,20 +324,10 @@ struct IndexedGatherOut {
 
 // Gather: partial sums of the 216 products (FP64 across the stencil rows) reduced with
 // shuffles inside each atom's lane group. Returns this thread's share of the self energy
-// -(a/sqrt(pi)) sum q^2. An atom takes 6 lanes, lane a the x index a of the stencil, so
-// that every other stencil index is a compile-time constant (registers, not local memory);
-// a warp holds 5 atoms (lanes 30, 31 idle). With 8 lanes per atom and the (x, y) row taken
-// from the lane index, the stencil weights went through local memory.
+// -(a/sqrt(pi)) sum q^2. An atom takes 6 lanes, lane a the x index a of the stencil; a warp
+// takes 5 atoms at a time (lanes 30, 31 idle) out of up to 10 staged stencils.
 constexpr int kGatherLanes = 6;
 constexpr int kGatherAtomsPerWarp = kWarp / kGatherLanes;
-
-template <class T>
-__device__ __forceinline__ T pick6(const T (&v)[6], int i) {
-  T r = v[0];
-#pragma unroll
-  for (int k = 1; k < 6; ++k) r = i == k ? v[k] : r;
-  return r;
-}
 
 // Sum over the 6 lanes 6k .. 6k + 5 of an atom, valid on lane 6k (fixed order).
 __device__ __forceinline__ double gather_lane_sum(double v) {
@@ -465,65 +337,94 @@ __device__ __forceinline__ double gather_lane_sum(double v) {
 }
 
 template <class T, class Atoms, class Out>
-__device__ __forceinline__ double gather_atoms(const Atoms &atoms, int64_t nthreads, const PmeShared &sh, int K,
+__device__ __forceinline__ double gather_atoms(const Atoms &atoms, int64_t n, const PmeShared &sh, int K,
                                                const T *Phi, double alpha, const Out &out, int64_t bid,
-                                               int64_t nblk) {
+                                               int64_t nblk, GatherStage<T> &S) {
   const double a_rpi = alpha / 1.7724538509055160273;
-  const int lw = threadIdx.x % kWarp;
-  const int slot = lw / kGatherLanes;     // atom of the warp (kGatherAtomsPerWarp: idle lane)
-  const int a = lw - slot * kGatherLanes;  // x index of the stencil
-  const int64_t wglob = (bid * blockDim.x + threadIdx.x) / kWarp;
-  const int64_t nwarps = nblk * blockDim.x / kWarp;
+  const int lane = threadIdx.x & 31;
+  const int slot = lane / kGatherLanes;     // atom of the round (kGatherAtomsPerWarp: idle lane)
+  const int a = lane - slot * kGatherLanes;  // x index of the stencil
+  const int64_t wg = (bid * blockDim.x + threadIdx.x) / kWarp;
+  const int64_t nw = nblk * blockDim.x / kWarp;
+  // one or two rounds of 5 atoms per pass, whichever fills the warps
+  const int apw = n > nw * kGatherAtomsPerWarp ? 2 * kGatherAtomsPerWarp : kGatherAtomsPerWarp;
   double e = 0.0;
-  for (int64_t wb = wglob * kGatherAtomsPerWarp; wb < nthreads; wb += nwarps * kGatherAtomsPerWarp) {
-    const int64_t t = wb + slot;
-    double rx = 0.0, ry = 0.0, rz = 0.0;
-    T q = T(0);
-    const bool ok = slot < kGatherAtomsPerWarp && t < nthreads && atoms.get(t, rx, ry, rz, q);
-    double phi = 0.0, du0 = 0.0, du1 = 0.0, du2 = 0.0;
-    if (ok) {
-      Stencil<T> s;
-      make_stencil<T>(rx, ry, rz, sh.recip, K, s);
-      int gx = s.g0[0] + a;
-      gx -= (gx >= K) ? K : 0;
-      // sums over the (y, z) plane at x index a: sum vy pz, sum dy pz, sum vy dz
-      double svp = 0.0, sdp = 0.0, svd = 0.0;
+  for (int64_t base = wg * apw; base < n; base += nw * apw) {
+    __syncwarp();  // every lane is done with the previous pass's stencils
+    T q = T(0);    // lane 3 k + d: charge of staged atom k, if there is one
+    bool has = false;
+    if (lane < 3 * apw) {
+      const int k = lane / 3, d = lane - 3 * k;
+      double rx, ry, rz;
+      has = base + k < n && atoms.get(base + k, rx, ry, rz, q);
+      if (has) {
+        SplinePoint2<T>(&p)[6] = S.p[k][d];
+        const double w = axis_points(rx, ry, rz, sh, K, d, [&](int i, int off) { p[i].off = off; });
+        T val[6], der[6];
+        bspline6<T>((T)w, val, der);
 #pragma unroll
-      for (int b = 0; b < 6; ++b) {
-        int gy = s.g0[1] + b;
-        gy -= (gy >= K) ? K : 0;
-        const int64_t row = ((int64_t)gx * K + gy) * K;
-        int gz = s.g0[2];
-        T pz = T(0), dz = T(0);
+        for (int i = 0; i < 6; ++i) {
+          p[i].w = val[i];
+          p[i].d = der[i];
+        }
+      }
+    }
+    const unsigned valid = __ballot_sync(kFull, has);
+    __syncwarp();
+#pragma unroll 1
+    for (int r = 0; r < apw; r += kGatherAtomsPerWarp) {
+      const int k = r + slot;
+      const bool ok = slot < kGatherAtomsPerWarp && ((valid >> (3 * min(k, 9))) & 1u);
+      const T qk = __shfl_sync(kFull, q, 3 * min(k, 9));
+      double phi = 0.0, du0 = 0.0, du1 = 0.0, du2 = 0.0;
+      if (ok) {
+        const auto &p = S.p[k];
+        const SplinePoint2<T> px = p[0][a];
+        T vz[6], dz6[6];
+        int oz[6];
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-          const T v = Phi[row + gz];
-          pz += v * s.val[2][c];
-          dz += v * s.der[2][c];
-          gz = (gz + 1 == K) ? 0 : gz + 1;
+          const SplinePoint2<T> z = p[2][c];
+          vz[c] = z.w;
+          dz6[c] = z.d;
+          oz[c] = z.off;
         }
-        svp += (double)s.val[1][b] * (double)pz;
-        sdp += (double)s.der[1][b] * (double)pz;
-        svd += (double)s.val[1][b] * (double)dz;
+        // sums over the (y, z) plane at x index a: sum vy pz, sum dy pz, sum vy dz
+        double svp = 0.0, sdp = 0.0, svd = 0.0;
+#pragma unroll
+        for (int b = 0; b < 6; ++b) {
+          const SplinePoint2<T> py = p[1][b];
+          const T *row = Phi + (px.off + py.off);
+          T pz = T(0), dz = T(0);
+#pragma unroll
+          for (int c = 0; c < 6; ++c) {
+            const T v = row[oz[c]];
+            pz += v * vz[c];
+            dz += v * dz6[c];
+          }
+          svp += (double)py.w * (double)pz;
+          sdp += (double)py.d * (double)pz;
+          svd += (double)py.w * (double)dz;
+        }
+        const double vx = (double)px.w, dx = (double)px.d;
+        phi = vx * svp;
+        du0 = dx * svp;
+        du1 = vx * sdp;
+        du2 = vx * svd;
       }
-      const double vx = (double)pick6(s.val[0], a), dx = (double)pick6(s.der[0], a);
-      phi = vx * svp;
-      du0 = dx * svp;
-      du1 = vx * sdp;
-      du2 = vx * svd;
-    }
-    phi = gather_lane_sum(phi);
-    du0 = gather_lane_sum(du0);
-    du1 = gather_lane_sum(du1);
-    du2 = gather_lane_sum(du2);
-    if (ok && a == 0) {
-      // u_d = m0 - frac_d + const, so d(stencil u)/dr_c = -recip[d][c]
-      const double qd = (double)q;
-      const double gxv = -qd * (du0 * sh.recip[0] + du1 * sh.recip[3] + du2 * sh.recip[6]);
-      const double gyv = -qd * (du0 * sh.recip[1] + du1 * sh.recip[4] + du2 * sh.recip[7]);
-      const double gzv = -qd * (du0 * sh.recip[2] + du1 * sh.recip[5] + du2 * sh.recip[8]);
-      out.put(t, phi - 2.0 * a_rpi * qd, gxv, gyv, gzv);
-      e -= a_rpi * qd * qd;
+      phi = gather_lane_sum(phi);
+      du0 = gather_lane_sum(du0);
+      du1 = gather_lane_sum(du1);
+      du2 = gather_lane_sum(du2);
+      if (ok && a == 0) {
+        // u_d = m0 - frac_d + const, so d(stencil u)/dr_c = -recip[d][c]
+        const double qd = (double)qk;
+        const double gxv = -qd * (du0 * sh.recip[0] + du1 * sh.recip[3] + du2 * sh.recip[6]);
+        const double gyv = -qd * (du0 * sh.recip[1] + du1 * sh.recip[4] + du2 * sh.recip[7]);
+        const double gzv = -qd * (du0 * sh.recip[2] + du1 * sh.recip[5] + du2 * sh.recip[8]);
+        out.put(base + k, phi - 2.0 * a_rpi * qd, gxv, gyv, gzv);
+        e -= a_rpi * qd * qd;
+      }
     }
   }
   return e;
@@ -535,9 +436,11 @@ __global__ void __launch_bounds__(kPmeBlock) pme_gather_kernel(Atoms atoms, int6
                                                                unsigned *ticket, double *e_self, const double *e_rec,
                                                                double e_scale, T *energy_out) {
   __shared__ PmeShared sh;
+  __shared__ GatherStage<T> st[kPmeBlock / kWarp];
   if (threadIdx.x == 0) load_pme_shared(box, K, sh);
   __syncthreads();
-  const double e = gather_atoms<T>(atoms, nthreads, sh, K, Phi, alpha, out, blockIdx.x, gridDim.x);
+  const double e = gather_atoms<T>(atoms, nthreads, sh, K, Phi, alpha, out, blockIdx.x, gridDim.x,
+                                   st[threadIdx.x >> 5]);
   const bool last = grid_sum<kPmeBlock>(e, partials, ticket, e_self, false);
   if (last && threadIdx.x == 0 && energy_out) energy_out[0] = (T)(e_scale * (*e_rec + *e_self));
 }
@@ -550,46 +453,73 @@ __global__ void __launch_bounds__(kPmeBlock) pme_gather_kernel(Atoms atoms, int6
 //   d/dx_i (sum_j u_j . dE/dx_j) = q_i recip^T (A v_i - B),  A_de = sum_g Phi H_de, B_d = sum_g psi G_d
 //   d/dq_i (sum_j u_j . dE/dx_j) = -v_i . C + sum_g psi theta_i,  C_d = sum_g Phi G_d
 // (the reciprocal energy is 1/2 Q.Phi; the self term has no coordinate dependence).
+// Staging and lanes as in spread_atoms; the products are FP64 in both precisions.
+struct DirStage {
+  SplinePoint2<double> p[kStencilAtoms][3][6];
+  double v[kStencilAtoms][3], q[kStencilAtoms];
+};
+
 template <class T>
 __global__ void __launch_bounds__(kPmeBlock) pme_spread_dir_kernel(PlainAtoms<T> atoms, const T *dir, int64_t n,
                                                                    const T *box, int K, typename Acc<T>::S *grid) {
   __shared__ PmeShared sh;
+  __shared__ DirStage st[kPmeBlock / kWarp];
   if (threadIdx.x == 0) load_pme_shared(box, K, sh);
   __syncthreads();
-  const int g = threadIdx.x % kLanesPerAtom;
-  const int64_t wglob = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
-  const int64_t nwarps = (int64_t)gridDim.x * blockDim.x / kWarp;
-  for (int64_t wb = wglob * kAtomsPerWarp; wb < n; wb += nwarps * kAtomsPerWarp) {
-    const int64_t t = wb + (threadIdx.x % kWarp) / kLanesPerAtom;
-    double rx, ry, rz;
-    T q;
-    if (t >= n || !atoms.get(t, rx, ry, rz, q)) continue;
-    const double ux = dir[3 * t], uy = dir[3 * t + 1], uz = dir[3 * t + 2];
-    const double v0 = sh.recip[0] * ux + sh.recip[1] * uy + sh.recip[2] * uz;
-    const double v1 = sh.recip[3] * ux + sh.recip[4] * uy + sh.recip[5] * uz;
-    const double v2 = sh.recip[6] * ux + sh.recip[7] * uy + sh.recip[8] * uz;
-    Stencil<T> s;
-    make_stencil<T>(rx, ry, rz, sh.recip, K, s);
-    for (int r = g; r < 36; r += kLanesPerAtom) {
-      const int a = r / 6, b = r % 6;
-      int gx = s.g0[0] + a, gy = s.g0[1] + b;
-      gx -= (gx >= K) ? K : 0;
-      gy -= (gy >= K) ? K : 0;
-      const double wx = s.val[0][a], dx = s.der[0][a], wy = s.val[1][b], dy = s.der[1][b];
-      const double c_val = -(double)q * (v0 * dx * wy + v1 * wx * dy);  // times val_z
-      const double c_der = -(double)q * v2 * wx * wy;                    // times der_z
-      const int64_t row = ((int64_t)gx * K + gy) * K;
-      int gz = s.g0[2];
+  DirStage &S = st[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  const int64_t wg = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kWarp;
+  const int64_t nw = (int64_t)gridDim.x * blockDim.x / kWarp;
+  const int apw = (int)min((int64_t)kStencilAtoms, max((int64_t)1, (n + nw - 1) / nw));
+  const int r0 = lane / 6, c = lane - 6 * r0;
+  for (int64_t base = wg * apw; base < n; base += nw * apw) {
+    __syncwarp();
+    const int left = (int)min((int64_t)apw, n - base);
+    if (lane < 3 * left) {
+      const int k = lane / 3, d = lane - 3 * k;
+      const int64_t t = base + k;
+      double rx, ry, rz;
+      T q;
+      atoms.get(t, rx, ry, rz, q);
+      const double ux = dir[3 * t], uy = dir[3 * t + 1], uz = dir[3 * t + 2];
+      S.v[k][d] = sh.recip[3 * d] * ux + sh.recip[3 * d + 1] * uy + sh.recip[3 * d + 2] * uz;
+      if (d == 0) S.q[k] = (double)q;
+      SplinePoint2<double>(&p)[6] = S.p[k][d];
+      const double w = axis_points(rx, ry, rz, sh, K, d, [&](int i, int off) { p[i].off = off; });
+      T val[6], der[6];
+      bspline6<T>((T)w, val, der);
 #pragma unroll
-      for (int c = 0; c < 6; ++c) {
-        Acc<T>::add(&grid[row + gz], c_val * (double)s.val[2][c] + c_der * (double)s.der[2][c]);
-        gz = (gz + 1 == K) ? 0 : gz + 1;
+      for (int i = 0; i < 6; ++i) {
+        p[i].w = (double)val[i];
+        p[i].d = (double)der[i];
       }
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int k = 0; k < left; ++k) {
+      if (lane >= 30) continue;
+      const auto &p = S.p[k];
+      const double v0 = S.v[k][0], v1 = S.v[k][1], v2 = S.v[k][2], nq = -S.q[k];
+      const SplinePoint2<double> pz = p[2][c], py = p[1][r0];
+      const auto add = [&](const SplinePoint2<double> &x, const SplinePoint2<double> &y) {
+        const double c_val = nq * (v0 * x.d * y.w + v1 * x.w * y.d);  // times val_z
+        const double c_der = nq * v2 * x.w * y.w;                      // times der_z
+        Acc<T>::add(&grid[x.off + y.off + pz.off], c_val * pz.w + c_der * pz.d);
+      };
+#pragma unroll
+      for (int a = 0; a < 6; ++a) add(p[0][a], py);
+      const SplinePoint2<double> p5 = p[1][5];
+      add(p[0][r0], p5);
+      if (r0 == 0) add(p[0][5], p5);
     }
   }
 }
 
-// Per atom: kc * d/dx_i and kc * d/dq_i of sum_j u_j . dE_rec/dx_j (kLanesPerAtom lanes per atom).
+// Per atom: kc * d/dx_i and kc * d/dq_i of sum_j u_j . dE_rec/dx_j (kLanesPerAtom lanes per atom,
+// lane g of them the (x, y) rows g, g + kLanesPerAtom, ...).
+constexpr int kLanesPerAtom = 8;
+constexpr int kAtomsPerWarp = kWarp / kLanesPerAtom;
+
 template <class T>
 __global__ void __launch_bounds__(kPmeBlock) pme_gather_hvp_kernel(PlainAtoms<T> atoms, const T *dir, int64_t n,
                                                                    const T *box, int K, const T *Phi, const T *Psi,
@@ -925,15 +855,12 @@ static __global__ void batch_fix_to_real_kernel(const BatchShape *shape, const u
 template <class T>
 __device__ __noinline__ void batch_spread_unit(const BatchSys *sys, const T *x, const T *q, const T *boxes,
                                                typename Acc<T>::S *grid, int sy, int bx, PmeShared &sh,
-                                               GroupStencil *st) {
+                                               SpreadStage<T> &st) {
   const BatchSys &b = sys[sy];
   if (threadIdx.x == 0) load_pme_shared(boxes + 9 * (int64_t)sy, b.K, sh);
   __syncthreads();
   PlainAtoms<T> atoms{x + 3 * b.atom_off, q + b.atom_off, b.natoms};
-  if constexpr (sizeof(T) == 4)
-    spread_groups(atoms, b.natoms, sh, b.K, grid + b.grid_off, bx, b.gather_blocks, st);
-  else
-    spread_atoms<T>(atoms, b.natoms, sh, b.K, grid + b.grid_off, bx, b.gather_blocks);
+  spread_atoms<T>(atoms, b.natoms, sh, b.K, grid + b.grid_off, bx, b.gather_blocks, st);
 }
 
 template <class T>
@@ -941,13 +868,12 @@ __global__ void __launch_bounds__(kPmeBlock, 4) batch_spread_kernel(const BatchS
                                                                  const T *x, const T *q, const T *boxes,
                                                                  typename Acc<T>::S *grid, unsigned *counter) {
   __shared__ PmeShared sh;
-  __shared__ GroupStencil st[sizeof(T) == 4 ? kPmeBlock / kWarp : 1][kSpreadGroup * kGroupsPerPass];
+  __shared__ SpreadStage<T> st[kPmeBlock / kWarp];
   // the gather's units (a system's atoms never outnumber its sorted slots)
   const int nsys = shape->nsys, units = shape->gather_units;
   for (int u = next_unit(counter); u < units; u = next_unit(counter)) {
     const int sy = unit_system<kUnitsGather>(sys, nsys, u);
-    batch_spread_unit<T>(sys, x, q, boxes, grid, sy, u - sys[sy].gather_off, sh,
-                         st[sizeof(T) == 4 ? threadIdx.x >> 5 : 0]);
+    batch_spread_unit<T>(sys, x, q, boxes, grid, sy, u - sys[sy].gather_off, sh, st[threadIdx.x >> 5]);
   }
 }
 
@@ -984,6 +910,7 @@ __global__ void __launch_bounds__(kPmeBlock, sizeof(T) == 4 ? 3 : 2) batch_gathe
                                                                  T *grad, double *partials, unsigned *tickets,
                                                                  double *energies, unsigned *counter) {
   __shared__ PmeShared sh;
+  __shared__ GatherStage<T> st[kPmeBlock / kWarp];
   const int nsys = shape->nsys, units = shape->gather_units;
   for (int u = next_unit(counter); u < units; u = next_unit(counter)) {
     const int sy = unit_system<kUnitsGather>(sys, nsys, u);
@@ -995,7 +922,8 @@ __global__ void __launch_bounds__(kPmeBlock, sizeof(T) == 4 ? 3 : 2) batch_gathe
     const int64_t nslots = b.ncl * kWarp;
     IndexedAtoms<T> atoms{x, q, slots, nslots};
     IndexedGatherOut<T> out{phi, grad, slots};
-    const double e = gather_atoms<T>(atoms, nslots, sh, b.K, Phi + b.grid_off, alpha, out, bx, b.gather_blocks);
+    const double e = gather_atoms<T>(atoms, nslots, sh, b.K, Phi + b.grid_off, alpha, out, bx, b.gather_blocks,
+                                     st[threadIdx.x >> 5]);
     grid_sum_n<kPmeBlock>(e, partials + (int64_t)kBatchPmeMaxBlocks * sy, tickets + 2 * sy + 1,
                           energies + 2 * sy + 1, false, bx, b.gather_blocks);
   }
@@ -1100,18 +1028,7 @@ int pme_grid_phase(const PmePlanImpl &p, const PmeLayout &L, char *ws, Atoms ato
   TFF_CUDA(cudaMemsetAsync(ws + L.zero_off, 0, L.zero_bytes, s));
   S *grid = reinterpret_cast<S *>(ws + L.fix);
   if (nthreads > 0) {
-    if constexpr (sizeof(T) == 4 && std::is_same<Atoms, PlainAtoms<float>>::value) {
-      // FP32 caller-order atoms: groups of consecutive atoms (bit-identical grid), one warp
-      // per group up to a few waves of blocks
-      const int64_t groups = (nthreads + kSpreadGroup - 1) / kSpreadGroup;
-      const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((groups * kWarp + kPmeBlock - 1) / kPmeBlock,
-                                                                 sm_count() * 8));
-      pme_spread_grouped_kernel<Atoms><<<nb, kPmeBlock, 0, s>>>(atoms, nthreads, box, p.K, grid);
-    } else {
-      const int64_t lanes = nthreads * kLanesPerAtom;
-      const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((lanes + kPmeBlock - 1) / kPmeBlock, sm_count() * 8));
-      pme_spread_kernel<T, Atoms><<<nb, kPmeBlock, 0, s>>>(atoms, nthreads, box, p.K, grid);
-    }
+    pme_spread_kernel<T, Atoms><<<pme_blocks(nthreads), kPmeBlock, 0, s>>>(atoms, nthreads, box, p.K, grid);
     TFF_LAUNCHED();
   }
   return pme_solve_phase<T>(p, L, ws, box, alpha, xmod, ymod, zmod, s, phi_grid);
@@ -1123,8 +1040,7 @@ int pme_gather_phase(const PmePlanImpl &p, const PmeLayout &L, char *ws, Atoms a
   double *partials = reinterpret_cast<double *>(ws + L.partials);
   unsigned *tickets = reinterpret_cast<unsigned *>(ws + L.tickets);
   double *energies = reinterpret_cast<double *>(ws + L.energies);
-  const int64_t lanes = (nthreads + kGatherAtomsPerWarp - 1) / kGatherAtomsPerWarp * kWarp;
-  const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((lanes + kPmeBlock - 1) / kPmeBlock, sm_count() * 8));
+  const int nb = pme_blocks((nthreads + kGatherAtomsPerWarp - 1) / kGatherAtomsPerWarp);
   pme_gather_kernel<T, Atoms, Out><<<nb, kPmeBlock, 0, s>>>(atoms, nthreads, box, p.K, phi_grid, alpha, out,
                                                             partials, tickets + 1, energies + 1, energies, e_scale,
                                                             energy_out);
