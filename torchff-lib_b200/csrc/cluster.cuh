@@ -28,6 +28,12 @@ namespace tff {
 // measured 3 % and 6 % slower at 9000 atoms and 4 % and 10 % slower at 300,000 atoms (more
 // items hold the SMs longer against the PME kernels of the other stream).
 constexpr int kItemTiles = 4;
+// Small single systems get smaller items: the neighbour search takes the item size total / kItemTarget
+// (between 1 and kItemTiles) for `total` listed cluster pairs, so that the warps a B200 holds of
+// the pair kernel take single clusters where there are few. With items of 4 a 648-atom box was 63
+// warps of four clusters one after another: pair kernel 31.7 -> 15 us. A target of 148 x 16 gave
+// 3,693 atoms items of 3, 5 % slower than items of 4.
+constexpr int kItemTarget = 148 * 8;
 // Consecutive clusters per super-cluster: the neighbour search screens a super-cluster's
 // union box first and tests its members only when that box is within the cutoff.
 constexpr int kSuper = 32;
@@ -41,6 +47,19 @@ template <> struct V4<double> { using type = D4; };
 
 __device__ __forceinline__ D4 make_v4(double x, double y, double z, double w) { return D4{x, y, z, w}; }
 __device__ __forceinline__ float4 make_v4(float x, float y, float z, float w) { return make_float4(x, y, z, w); }
+
+// Item size of a single system with `total` listed cluster pairs. FP64 keeps full items: there each
+// item's energy is one more FP64 atomic, and their order shows in the last digits of the total.
+template <class T>
+__device__ __forceinline__ int item_size(int total) {
+  return sizeof(T) == 4 ? min(max(total / kItemTarget, 1), kItemTiles) : kItemTiles;
+}
+
+// Most work items of `nclusters` lists of at most `cap` clusters (see kItemTarget).
+inline int64_t item_capacity(int64_t nclusters, int64_t cap) {
+  return std::max(nclusters * ((cap + kItemTiles - 1) / kItemTiles),
+                  std::min(nclusters * cap, (int64_t)kItemTiles * kItemTarget));
+}
 
 struct ClusterLayout {
   int nc = 1, bits = 0;
@@ -98,7 +117,7 @@ inline ClusterLayout cluster_layout(int dtype, int64_t natoms, int cap) {
   L.nbr = (c.off + 255) & ~size_t(255); c.take<int>((size_t)L.nclusters * cap);
   L.ncount = (c.off + 255) & ~size_t(255); c.take<int>(L.nclusters);
   L.itemoff = (c.off + 255) & ~size_t(255); c.take<int>(L.nclusters + 1);
-  L.items = (c.off + 255) & ~size_t(255); c.take<int>((size_t)L.nclusters * ((cap + kItemTiles - 1) / kItemTiles));
+  L.items = (c.off + 255) & ~size_t(255); c.take<int>((size_t)item_capacity(L.nclusters, cap));
   L.boxinfo = (c.off + 255) & ~size_t(255); c.take<double>(32);
   L.bytes = c.bytes();
   return L;
@@ -144,7 +163,7 @@ struct ClusterData {
   using V = typename V4<T>::type;
   unsigned *keys, *hist, *fill, *status;
   int *tmp, *sidx, *inv, *nbr, *ncount;
-  int *itemoff;  // work items of the tile kernel: prefix sums of ceil(ncount / kItemTiles)
+  int *itemoff;  // work items of the tile kernel: prefix sums of ceil(ncount / item size)
   int *items;    // owning cluster of each work item
   V *pos, *frac, *bc, *bh;
   V *sbc, *sbh;     // union boxes of kSuper consecutive clusters (fractional centre, half extent)
@@ -583,17 +602,91 @@ __global__ void __launch_bounds__(kBatchSortThreads) batch_sort_kernel(const T *
   }
 }
 
-// One warp per cluster: bounding box in fractional coordinates. The box is taken around
+// Bounding box of cluster c in fractional coordinates, by one warp. The box is taken around
 // the first atom's image so that a cluster straddling the periodic boundary stays compact,
 // and the cluster's positions are rewritten as that same contiguous image (anchor +
-// nearest-image offset), so that one periodic shift serves a whole cluster pair.
-// A block of kSuper warps covers one super-cluster and, once its member boxes are known,
-// takes their union around the first member's centre (members shifted to their nearest
-// image of it) and widens it by 1e-5 to cover the rounding of centres to T.
+// nearest-image offset), so that one periodic shift serves a whole cluster pair. `m`: the box. On
+// lane 0 stores the box in d.bc, d.bh and the centre in `centre`; returns the half extents.
+template <class T>
+__device__ __forceinline__ typename ClusterData<T>::V cluster_box(const ClusterData<T> &d, const double *m, int64_t c,
+                                                                  int lane, typename ClusterData<T>::V &centre) {
+  const int64_t s = c * kWarp + lane;
+  const bool valid = d.sidx[s] >= 0;
+  auto f = d.frac[s];
+  T fx = f.x, fy = f.y, fz = f.z;
+  const T ax = __shfl_sync(kFull, fx, 0), ay = __shfl_sync(kFull, fy, 0), az = __shfl_sync(kFull, fz, 0);
+  fx -= ax; fy -= ay; fz -= az;
+  fx -= floor(fx + T(0.5)); fy -= floor(fy + T(0.5)); fz -= floor(fz + T(0.5));
+  if (valid) {
+    const double ux = (double)ax + (double)fx, uy = (double)ay + (double)fy, uz = (double)az + (double)fz;
+    auto p = d.pos[s];
+    p.x = (T)(ux * m[0] + uy * m[3] + uz * m[6]);
+    p.y = (T)(ux * m[1] + uy * m[4] + uz * m[7]);
+    p.z = (T)(ux * m[2] + uy * m[5] + uz * m[8]);
+    d.pos[s] = p;
+  }
+  T lo[3] = {valid ? fx : T(1e30), valid ? fy : T(1e30), valid ? fz : T(1e30)};
+  T hi[3] = {valid ? fx : T(-1e30), valid ? fy : T(-1e30), valid ? fz : T(-1e30)};
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      lo[k] = min(lo[k], __shfl_xor_sync(kFull, lo[k], o));
+      hi[k] = max(hi[k], __shfl_xor_sync(kFull, hi[k], o));
+    }
+  }
+  const auto cc = make_v4(ax + T(0.5) * (lo[0] + hi[0]), ay + T(0.5) * (lo[1] + hi[1]), az + T(0.5) * (lo[2] + hi[2]),
+                          T(0));
+  const auto hh = make_v4(T(0.5) * (hi[0] - lo[0]), T(0.5) * (hi[1] - lo[1]), T(0.5) * (hi[2] - lo[2]), T(0));
+  if (lane == 0) {
+    d.bc[c] = cc;
+    d.bh[c] = hh;
+    centre = cc;
+  }
+  return hh;
+}
+
+// Union box of super-cluster S, by one warp: lane l holds member l's centre and half extents
+// (members lanes), ref the first member's centre.
+template <class T>
+__device__ __forceinline__ void super_box(const ClusterData<T> &d, int64_t S, int members, int lane,
+                                          typename ClusterData<T>::V c, typename ClusterData<T>::V h,
+                                          typename ClusterData<T>::V ref) {
+  const bool v = lane < members;
+  const double cs[3] = {(double)c.x, (double)c.y, (double)c.z}, hs[3] = {(double)h.x, (double)h.y, (double)h.z};
+  const double rs[3] = {(double)ref.x, (double)ref.y, (double)ref.z};
+  double lo[3], hi[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    double u = v ? cs[k] - rs[k] : 0.0;
+    u -= floor(u + 0.5);
+    lo[k] = v ? rs[k] + u - hs[k] : 1e30;
+    hi[k] = v ? rs[k] + u + hs[k] : -1e30;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      lo[k] = fmin(lo[k], __shfl_xor_sync(kFull, lo[k], o));
+      hi[k] = fmax(hi[k], __shfl_xor_sync(kFull, hi[k], o));
+    }
+  }
+  if (lane == 0) {
+    d.sbc[S] = make_v4((T)(0.5 * (lo[0] + hi[0])), (T)(0.5 * (lo[1] + hi[1])), (T)(0.5 * (lo[2] + hi[2])), T(0));
+    d.sbh[S] = make_v4((T)(0.5 * (hi[0] - lo[0]) + 1e-5), (T)(0.5 * (hi[1] - lo[1]) + 1e-5),
+                       (T)(0.5 * (hi[2] - lo[2]) + 1e-5), T(0));
+  }
+}
+
+// One warp per cluster: its bounding box (cluster_box). A block of kSuper warps covers one
+// super-cluster and, once its member boxes are known, takes their union around the first
+// member's centre (members shifted to their nearest image of it) and widens it by 1e-5 to cover
+// the rounding of centres to T.
 template <class T>
 __global__ void __launch_bounds__(kWarp * kSuper) cluster_bounds_kernel(ClusterData<T> d) {
   pdl_enter();
-  __shared__ double s_box[kSuper][6];
+  using V = typename ClusterData<T>::V;
+  __shared__ V s_c[kSuper], s_h[kSuper];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int64_t nsuper = d.n_super();
   for (int64_t S = blockIdx.x; S < nsuper; S += gridDim.x) {
@@ -609,67 +702,13 @@ __global__ void __launch_bounds__(kWarp * kSuper) cluster_bounds_kernel(ClusterD
     const double *m = d.info(sy);
     const int64_t c = first + w;
     if (c < last) {
-      const int64_t s = c * kWarp + lane;
-      const bool valid = d.sidx[s] >= 0;
-      auto f = d.frac[s];
-      T fx = f.x, fy = f.y, fz = f.z;
-      const T ax = __shfl_sync(kFull, fx, 0), ay = __shfl_sync(kFull, fy, 0), az = __shfl_sync(kFull, fz, 0);
-      fx -= ax; fy -= ay; fz -= az;
-      fx -= floor(fx + T(0.5)); fy -= floor(fy + T(0.5)); fz -= floor(fz + T(0.5));
-      if (valid) {
-        const double ux = (double)ax + (double)fx, uy = (double)ay + (double)fy, uz = (double)az + (double)fz;
-        auto p = d.pos[s];
-        p.x = (T)(ux * m[0] + uy * m[3] + uz * m[6]);
-        p.y = (T)(ux * m[1] + uy * m[4] + uz * m[7]);
-        p.z = (T)(ux * m[2] + uy * m[5] + uz * m[8]);
-        d.pos[s] = p;
-      }
-      T lo[3] = {valid ? fx : T(1e30), valid ? fy : T(1e30), valid ? fz : T(1e30)};
-      T hi[3] = {valid ? fx : T(-1e30), valid ? fy : T(-1e30), valid ? fz : T(-1e30)};
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          lo[k] = min(lo[k], __shfl_xor_sync(kFull, lo[k], o));
-          hi[k] = max(hi[k], __shfl_xor_sync(kFull, hi[k], o));
-        }
-      }
-      if (lane == 0) {
-        const auto cc = make_v4(ax + T(0.5) * (lo[0] + hi[0]), ay + T(0.5) * (lo[1] + hi[1]),
-                                az + T(0.5) * (lo[2] + hi[2]), T(0));
-        const auto hh = make_v4(T(0.5) * (hi[0] - lo[0]), T(0.5) * (hi[1] - lo[1]), T(0.5) * (hi[2] - lo[2]), T(0));
-        d.bc[c] = cc;
-        d.bh[c] = hh;
-        s_box[w][0] = cc.x; s_box[w][1] = cc.y; s_box[w][2] = cc.z;
-        s_box[w][3] = hh.x; s_box[w][4] = hh.y; s_box[w][5] = hh.z;
-      }
+      const V h = cluster_box(d, m, c, lane, s_c[w]);
+      if (lane == 0) s_h[w] = h;
     }
     __syncthreads();
-    if (w == 0) {
-      const bool v = first + lane < last;
-      double lo[3], hi[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const double ref = s_box[0][k];
-        double u = v ? s_box[lane][k] - ref : 0.0;
-        u -= floor(u + 0.5);
-        lo[k] = v ? ref + u - s_box[lane][3 + k] : 1e30;
-        hi[k] = v ? ref + u + s_box[lane][3 + k] : -1e30;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          lo[k] = fmin(lo[k], __shfl_xor_sync(kFull, lo[k], o));
-          hi[k] = fmax(hi[k], __shfl_xor_sync(kFull, hi[k], o));
-        }
-      }
-      if (lane == 0) {
-        d.sbc[S] = make_v4((T)(0.5 * (lo[0] + hi[0])), (T)(0.5 * (lo[1] + hi[1])), (T)(0.5 * (lo[2] + hi[2])), T(0));
-        d.sbh[S] = make_v4((T)(0.5 * (hi[0] - lo[0]) + 1e-5), (T)(0.5 * (hi[1] - lo[1]) + 1e-5),
-                           (T)(0.5 * (hi[2] - lo[2]) + 1e-5), T(0));
-      }
-    }
+    if (w == 0)
+      super_box(d, S, (int)(last - first), lane, first + lane < last ? s_c[lane] : V{},
+                first + lane < last ? s_h[lane] : V{}, s_c[0]);
     __syncthreads();
   }
 }
@@ -810,12 +849,13 @@ __global__ void cluster_neighbors_kernel(ClusterData<T> d, double rc, int half) 
     }
   }
   // The last block to finish turns the counts into work-item offsets (exclusive prefix
-  // sums of ceil(count / kItemTiles)); status[1] is the block ticket (zeroed per build).
+  // sums of ceil(count / item size)); status[1] is the block ticket (zeroed per build).
   // The item -> cluster table is filled by the sorted-parameter kernel that follows.
   __shared__ bool s_last;
-  __shared__ int s_warp[32];
+  __shared__ int s_warp[32], s_size;
   __syncthreads();
   if (threadIdx.x == 0) {
+    s_size = 0;
     __threadfence();
     s_last = atomicAdd(&d.status[1], 1u) == gridDim.x - 1;
   }
@@ -825,8 +865,15 @@ __global__ void cluster_neighbors_kernel(ClusterData<T> d, double rc, int half) 
   const int64_t n = ncl;
   const int64_t per = (n + blockDim.x - 1) / blockDim.x;
   const int64_t beg = min((int64_t)threadIdx.x * per, n), end = min(beg + per, n);
+  int total = 0;
+  for (int64_t k = beg; k < end; ++k) total += __ldcg(&d.ncount[k]);
+  total = __reduce_add_sync(kFull, total);
+  if (lane == 0) atomicAdd(&s_size, total);
+  __syncthreads();
+  // a batch keeps the full size: a system's FP32 sums over an item then do not depend on the batch
+  const int size = d.shape ? kItemTiles : item_size<T>(s_size);
   int sum = 0;
-  for (int64_t k = beg; k < end; ++k) sum += (__ldcg(&d.ncount[k]) + kItemTiles - 1) / kItemTiles;
+  for (int64_t k = beg; k < end; ++k) sum += (__ldcg(&d.ncount[k]) + size - 1) / size;
   int incl = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -850,9 +897,155 @@ __global__ void cluster_neighbors_kernel(ClusterData<T> d, double rc, int half) 
   int run = s_warp[w] + incl - sum;
   for (int64_t k = beg; k < end; ++k) {
     d.itemoff[k] = run;
-    run += (__ldcg(&d.ncount[k]) + kItemTiles - 1) / kItemTiles;
+    run += (__ldcg(&d.ncount[k]) + size - 1) / size;
   }
   if (threadIdx.x == blockDim.x - 1) d.itemoff[n] = run;
+}
+
+// Steps 1-6 of a small system in one launch of one block: a thread per atom, a warp per cluster.
+// Up to kSmallAtoms atoms (32 clusters, one super-cluster) the seven launches of the general build
+// are latency from end to end (34 us of kernels for 648 atoms; this one 8.8 us); the sort order,
+// boxes, lists and work items are the same.
+constexpr int kSmallAtoms = 1024;
+constexpr int kSmallKeys = 512;  // the cell grid of 1024 atoms: 5 cells per side, 3 bits per axis
+
+template <class T>
+__global__ void __launch_bounds__(kSmallAtoms) small_build_kernel(const T *x, const T *q, const T *box,
+                                                                  ClusterData<T> d, double rc, int half,
+                                                                  unsigned long long *zero, int64_t nzero) {
+  pdl_enter();
+  using V = typename ClusterData<T>::V;
+  __shared__ double s_info[kInfoStride];
+  __shared__ unsigned s_hist[kSmallKeys + 1], s_fill[kSmallKeys];
+  __shared__ unsigned short s_order[kSmallAtoms];
+  __shared__ unsigned s_warp[kWarp];
+  __shared__ V s_c[kWarp], s_h[kWarp];
+  __shared__ int s_count[kWarp];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int n = (int)d.natoms, ncl = (int)d.nclusters, nkeys = 1 << (3 * d.bits);
+  // the atom's coordinates, while thread 0 works out the box
+  double r[3] = {0.0, 0.0, 0.0};
+  T qa = T(0);
+  if (tid < n) {
+    r[0] = x[3 * tid];
+    r[1] = x[3 * tid + 1];
+    r[2] = x[3 * tid + 2];
+    if (q) qa = q[tid];
+  }
+  if (tid == 0) write_box_info(box, s_info);
+  for (int k = tid; k <= nkeys; k += blockDim.x) s_hist[k] = 0u;
+  for (int k = tid; k < nkeys; k += blockDim.x) s_fill[k] = 0u;
+  if (tid < 64) d.status[tid] = 0u;
+  for (int64_t k = tid; k < nzero; k += blockDim.x) zero[k] = 0ull;
+  __syncthreads();
+  if (tid < kInfoStride) d.boxinfo[tid] = s_info[tid];
+  const double *m = s_info, *inv = s_info + 9;
+  double f[3];
+  unsigned key = 0u;
+  if (tid < n) {
+    unsigned cell[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      double v = r[0] * inv[c] + r[1] * inv[3 + c] + r[2] * inv[6 + c];
+      v -= floor(v);
+      if (v >= 1.0) v = 0.0;  // guards rounding of tiny negatives
+      f[c] = v;
+      cell[c] = min((unsigned)(v * d.nc), (unsigned)(d.nc - 1));
+    }
+    key = hilbert_key(cell[0], cell[1], cell[2], d.bits);
+    atomicAdd(&s_hist[key], 1u);
+  }
+  __syncthreads();
+  // exclusive scan of the histogram, one key per thread
+  {
+    const unsigned v = tid < nkeys ? s_hist[tid] : 0u;
+    unsigned incl = v;
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+      const unsigned y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == kWarp - 1) s_warp[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+      const unsigned t = s_warp[lane];
+      unsigned ti = t;
+#pragma unroll
+      for (int o = 1; o < kWarp; o <<= 1) {
+        const unsigned y = __shfl_up_sync(kFull, ti, o);
+        if (lane >= o) ti += y;
+      }
+      s_warp[lane] = ti - t;
+    }
+    __syncthreads();
+    if (tid < nkeys) s_hist[tid] = s_warp[w] + incl - v;
+    if (tid == 0) s_hist[nkeys] = (unsigned)n;
+  }
+  __syncthreads();
+  if (tid < n) s_order[s_hist[key] + atomicAdd(&s_fill[key], 1u)] = (unsigned short)tid;
+  __syncthreads();
+  // an atom's slot is its rank (by atom index) inside its bucket
+  if (tid < n) {
+    const int b0 = (int)s_hist[key], b1 = (int)s_hist[key + 1];
+    int slot = b0;
+    for (int k = b0; k < b1; ++k) slot += s_order[k] < tid ? 1 : 0;
+    const double wx = f[0] * m[0] + f[1] * m[3] + f[2] * m[6];
+    const double wy = f[0] * m[1] + f[1] * m[4] + f[2] * m[7];
+    const double wz = f[0] * m[2] + f[1] * m[5] + f[2] * m[8];
+    d.pos[slot] = make_v4((T)wx, (T)wy, (T)wz, qa);
+    d.frac[slot] = make_v4((T)f[0], (T)f[1], (T)f[2], T(0));
+    d.sidx[slot] = tid;
+    d.inv[tid] = slot;
+  } else if (tid < d.npad) {
+    d.sidx[tid] = -1;
+    d.pos[tid] = make_v4(T(0), T(0), T(0), T(0));
+    d.frac[tid] = make_v4(T(0), T(0), T(0), T(0));
+  }
+  __syncthreads();
+  if (w < ncl) {
+    const V h = cluster_box(d, m, w, lane, s_c[w]);
+    if (lane == 0) s_h[w] = h;
+  }
+  __syncthreads();
+  if (w == 0) super_box(d, 0, ncl, lane, lane < ncl ? s_c[lane] : V{}, lane < ncl ? s_h[lane] : V{}, s_c[0]);
+  // neighbour lists: lane J against cluster w
+  int count = 0;
+  if (w < ncl) {
+    BoxTestF bt{};
+    if constexpr (sizeof(T) == 4) bt = box_test_f(s_info, rc);
+    bool ok = lane < (half ? w + 1 : ncl);
+    if (ok) {
+      if constexpr (sizeof(T) == 4)
+        ok = boxes_may_interact_f(s_c[w], s_h[w], s_c[lane], s_h[lane], bt);
+      else
+        ok = clusters_may_interact<T>(s_c[w], s_h[w], s_c[lane], s_h[lane], s_info, rc);
+    }
+    const unsigned mm = __ballot_sync(kFull, ok);
+    const int at = __popc(mm & ((1u << lane) - 1u));
+    if (ok && at < d.cap) d.nbr[(int64_t)w * d.cap + at] = lane;
+    count = min(__popc(mm), d.cap);
+    if (lane == 0) {
+      d.ncount[w] = count;
+      if (__popc(mm) > d.cap) atomicOr(&d.status[0], 1u);
+    }
+  }
+  if (lane == 0) s_count[w] = count;
+  __syncthreads();
+  if (w == 0) {
+    const int c = s_count[lane], size = item_size<T>(__reduce_add_sync(kFull, c)), items = (c + size - 1) / size;
+    int incl = items;
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+      const int y = __shfl_up_sync(kFull, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane < ncl) d.itemoff[lane] = incl - items;
+    if (lane == kWarp - 1) d.itemoff[ncl] = incl;
+  }
+}
+
+inline bool small_build(const ClusterLayout &L) {
+  return L.natoms > 0 && L.natoms <= kSmallAtoms && L.nkeys <= kSmallKeys;
 }
 
 // Host driver for steps 1-6 on `stream`. `zero` (`zero_bytes`, a multiple of 8) is cleared
@@ -862,6 +1055,9 @@ int build_clusters(const ClusterLayout &L, const ClusterData<T> &d, void *ws, co
                    const T *box, double rc, int half, cudaStream_t s, void *zero = nullptr, size_t zero_bytes = 0,
                    bool pdl = false) {
   const int sms = sm_count();
+  if (small_build(L))
+    return launch_k(false, small_build_kernel<T>, 1, kSmallAtoms, 0, s, x, q, box, d, rc, half,
+                    static_cast<unsigned long long *>(zero), (int64_t)(zero_bytes / 8));
   const int64_t nz = (int64_t)(L.zero_bytes / 8);
   const int nb_zero = (int)std::max<int64_t>(1, std::min<int64_t>((nz + 1023) / 1024, sms));
   int st = launch_k(false, box_info_kernel<T>, nb_zero, 256, 0, s, box, d.boxinfo,

@@ -172,7 +172,7 @@ int system_eval_impl(tff_system sys, const T *x, const T *box, double *energy, T
     A.energies = energies;
     // work items are only known on the device: size the grid for the largest possible
     // count (every cluster with a full list), capped at a few waves of the SMs
-    const int64_t max_items = sys->cl.nclusters * ((sys->cl.cap + kItemTiles - 1) / kItemTiles);
+    const int64_t max_items = item_capacity(sys->cl.nclusters, sys->cl.cap);
     if ((st = launch_real_space<T>(pdl, max_items, sms, s, A)) != TFF_OK) return st;
   }
   if ((st = mark(2, s)) != TFF_OK) return st;
@@ -312,7 +312,7 @@ int system_grad_impl(tff_system sys, const T *x, const T *box, const T *dir, dou
     A.alpha = sys->desc.ewald_alpha;
     A.kc = sys->desc.coul_constant;
     A.energies = energies;
-    const int64_t max_items = sys->cl.nclusters * ((sys->cl.cap + kItemTiles - 1) / kItemTiles);
+    const int64_t max_items = item_capacity(sys->cl.nclusters, sys->cl.cap);
     constexpr int NW = TileCfg<T, MODE>::NW;
     const int nbt = (int)std::max<int64_t>(1, std::min<int64_t>((max_items + NW - 1) / NW, (int64_t)sms * 48 / NW));
     tile_kernel<T, MODE><<<nbt, NW * kWarp, 0, s>>>(A);
@@ -791,8 +791,9 @@ int tff_system_hvp(tff_system sys, const void *coords, const void *box, const vo
 
 int tff_system_kernel_launches(tff_system sys) {
   if (!sys) return 0;
-  // cluster build 7 + sorted params 1 + tile 1 + finalize 1; PME: spread, [to_real], convolve, gather
-  int k = 10;
+  // cluster build 7 (1 for a small system) + sorted params 1 + tile 1 + finalize 1; PME: spread,
+  // [to_real], convolve, gather
+  int k = small_build(sys->cl) ? 4 : 10;
   if (sys->pme) k += sys->desc.dtype == TFF_F32 ? 4 : 3;
   return k;
 }
