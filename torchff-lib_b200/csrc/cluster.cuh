@@ -456,9 +456,9 @@ __global__ void sort_buckets_kernel(const T *x, const T *q, int64_t nkeys, Clust
 }
 
 // Batch mode, steps 1-5 in one launch: one block per system bins its atoms on the
-// system's own Hilbert-ordered cell grid in shared memory (counting sort, then an
-// insertion sort of each bucket by atom index, which makes the order deterministic and
-// equal to the single-system sort), writes the sorted SoA with padding to whole clusters
+// system's own Hilbert-ordered cell grid in shared memory (counting sort, then each atom's
+// rank by index in its bucket, which makes the order deterministic and equal to the
+// single-system sort), writes the sorted SoA with padding to whole clusters
 // and the cluster / super-cluster owners, and zeroes the energy kernel's accumulators of
 // those slots (acc: dE/dx of slots_cap slots, then dE/dq). The system count comes from
 // d.shape. Limits: kBatchMaxAtoms atoms and
@@ -494,8 +494,13 @@ __global__ void __launch_bounds__(kBatchSortThreads) batch_sort_kernel(const T *
     for (int k = tid; k < nkeys; k += blockDim.x) fill[k] = 0u;
     __syncthreads();
     const double *inv = s_info + 9;
+    // the next atom's coordinates load while this one's key is worked out
+    T nx = T(0), ny = T(0), nz = T(0);
+    if (tid < n) nx = xs[3 * tid], ny = xs[3 * tid + 1], nz = xs[3 * tid + 2];
     for (int t = tid; t < n; t += blockDim.x) {
-      const double rx = xs[3 * t], ry = xs[3 * t + 1], rz = xs[3 * t + 2];
+      const double rx = nx, ry = ny, rz = nz;
+      const int tn = t + (int)blockDim.x;
+      if (tn < n) nx = xs[3 * tn], ny = xs[3 * tn + 1], nz = xs[3 * tn + 2];
       unsigned cell[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -548,33 +553,38 @@ __global__ void __launch_bounds__(kBatchSortThreads) batch_sort_kernel(const T *
       order[hist[key] + atomicAdd(&fill[key], 1u)] = (unsigned short)t;
     }
     __syncthreads();
-    for (int k = tid; k < nkeys; k += blockDim.x) {
-      const int b0 = (int)hist[k], b1 = (int)hist[k + 1];
-      for (int i = b0 + 1; i < b1; ++i) {
-        const unsigned short v = order[i];
-        int j = i - 1;
-        while (j >= b0 && order[j] > v) {
-          order[j + 1] = order[j];
-          --j;
-        }
-        order[j + 1] = v;
-      }
-    }
-    __syncthreads();
     const double *m = s_info;
     const int64_t base = b.cl_off * kWarp;
     const int npad = (int)(b.ncl * kWarp);
+    // an atom's slot is its rank (by atom index) inside its bucket, counted by its own thread (one
+    // thread sorting a bucket by insertion took as long as the rest: 65 -> 52 us for 60 systems of
+    // 250 to 4,000 waters); the next position's atom loads meanwhile
+    int tn = tid < n ? (int)order[tid] : 0;
+    T nqx = T(0), nqy = T(0), nqz = T(0);
+    if (tid < n) nqx = xs[3 * tn], nqy = xs[3 * tn + 1], nqz = xs[3 * tn + 2];
     for (int p = tid; p < npad; p += blockDim.x) {
-      const int64_t slot = base + p;
+      const int t = tn;
+      const double rx = nqx, ry = nqy, rz = nqz;
+      const int pn = p + (int)blockDim.x;
+      if (pn < n) {
+        tn = order[pn];
+        nqx = xs[3 * tn], nqy = xs[3 * tn + 1], nqz = xs[3 * tn + 2];
+      }
+      int64_t slot = base + p;
+      if (p < n) {
+        const unsigned key = lkey[t];
+        const int b0 = (int)hist[key], b1 = (int)hist[key + 1];
+        int rank = 0;
+        for (int k = b0; k < b1; ++k) rank += order[k] < t ? 1 : 0;
+        slot = base + b0 + rank;
+      }
       // the energy kernel's accumulators of the slot: dE/dx (3 per slot), then dE/dq
       acc[3 * slot] = 0ull;
       acc[3 * slot + 1] = 0ull;
       acc[3 * slot + 2] = 0ull;
       acc[3 * slots_cap + slot] = 0ull;
       if (p < n) {
-        const int t = order[p];
         const int64_t a = b.atom_off + t;
-        const double rx = xs[3 * t], ry = xs[3 * t + 1], rz = xs[3 * t + 2];
         double f[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
