@@ -257,7 +257,10 @@ class _SystemGradFn(torch.autograd.Function):
     def forward(ctx, coords, box, q, sig, eps, gx, gq, gs, ge, system):
         ctx.save_for_backward(coords, box, q, sig, eps)
         ctx.system = system
-        return gx.clone(), gq.clone(), gs.clone(), ge.clone()
+        # cotangents nothing flowed into arrive as None, not as zeros that have to be read back
+        ctx.set_materialize_grads(False)
+        # only _SystemEnergyFn.backward calls this, and hands out products of these
+        return gx, gq, gs, ge
 
     @staticmethod
     def backward(ctx, vx, vq, vs, ve):
