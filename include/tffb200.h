@@ -411,9 +411,8 @@ int tff_system_kernel_launches(tff_system sys);
  * precision: bit-identical whatever else is in the batch). Same physics as tff_system_*;
  * cutoff, Ewald alpha and the Coulomb constant are shared by the batch.
  * Per system: 1 <= natoms <= 16384, 6 <= K <= 96 (TFF_F32) or 64 (TFF_F64). The
- * reciprocal-space transforms of a batch are a direct 3-D DFT of every grid (one launch per
- * axis pass for all sizes), not cuFFT; results match the single-system (cuFFT) path to FP
- * rounding.
+ * reciprocal-space transforms take all grid sizes in the same three launches, with the
+ * arithmetic of a single system's.
  * --------------------------------------------------------------------------- */
 typedef struct tff_batch_s *tff_batch;
 
@@ -439,9 +438,9 @@ int tff_batch_destroy(tff_batch batch);
  * their own system, -1 padded; out: energies (nsys) float64, forces (sum natoms, 3) in the batch dtype.
  * The host part (system table, work-unit offsets) runs in the call; the call returns once
  * the work is enqueued. One evaluation at a time per batch object and stream.
- * Every launch shape of the device part depends on the batch's capacity and the DFT size
+ * Every launch shape of the device part depends on the batch's capacity and the transform size
  * class (grid sides up to 52, or larger) alone; the composition is uploaded with the
- * system table. So when a call repeats the previous call's device pointers and DFT class,
+ * system table. So when a call repeats the previous call's device pointers and transform class,
  * the device part is captured in a CUDA graph, and later calls with those pointers and
  * that class replay it whatever systems they hold (up to 8 graphs per batch object). */
 int tff_batch_eval(tff_batch batch, int nsys, const int64_t *natoms, const int *pme_grid, const void *coords,

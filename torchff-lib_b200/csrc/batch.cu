@@ -4,16 +4,15 @@
 //   main stream : batch_sort (one block per system: its own box facts and Hilbert cell
 //                 grid) -> cluster bounds -> cluster neighbours -> sorted parameters ->
 //                 tile kernel -> [join] -> finalize (forces, one energy per system)
-//   PME stream  : spread (blockIdx.y = system) -> [fixed point -> FP32] -> 3-D real DFT
-//                 (three axis passes over all systems) -> convolution -> inverse DFT
-//                 (three passes) -> gather
+//   PME stream  : spread -> forward planes -> solve rows -> inverse planes (pme_fft.cuh, over
+//                 the planes of all systems) -> gather
 //
 // Systems are laid out one after another in every array; the cluster lists never leave a
 // system, and every per-system reduction runs over a block count that depends on that
 // system alone, so a system's result does not depend on what else is in the batch. The
-// reciprocal-space transforms are the batched direct DFT of pme.cuh (one launch per axis
-// pass for all grid sizes): cuFFT transforms grids of one size per plan, and a batch of
-// a few hundred sizes would need hundreds of plans and launches per evaluation.
+// reciprocal-space transforms take every grid size in the same launches: cuFFT transforms
+// grids of one size per plan, and a batch of a few hundred sizes would need hundreds of plans and
+// launches per evaluation.
 #include <algorithm>
 #include <cstring>
 #include <cmath>
@@ -25,12 +24,11 @@
 namespace tff {
 namespace {
 
-// Largest PME grid side of a batch: the DFT stages two K x K planes in shared memory.
+// Largest PME grid side of a batch: a transform stages two K x K planes in shared memory.
 constexpr int kBatchMaxK = 96;
 constexpr int kBatchMaxK64 = 64;
 
-// Grid distances inside the batch: every real grid starts on a 256-byte boundary and every
-// complex grid on a 256-byte (FP32) boundary, as cuFFT wants aligned transform inputs.
+// Grid distances inside the batch: every grid starts on a 256-byte boundary.
 inline int64_t real_dist(int K) { return ((int64_t)K * K * K + 63) / 64 * 64; }
 inline int64_t cplx_dist(int K) { return ((int64_t)K * K * (K / 2 + 1) + 31) / 32 * 32; }
 
@@ -41,10 +39,18 @@ inline int moduli_offset(int K) {
   return off;
 }
 
+// Offset of grid side K's transform tables, K up to kBatchMaxK + 1.
+inline int table_offset(int K) {
+  static const std::vector<int> off = [] {
+    std::vector<int> o(kBatchMaxK + 2, 0);
+    for (int k = 6; k <= kBatchMaxK; ++k) o[k + 1] = o[k] + k;
+    return o;
+  }();
+  return off[K];
+}
+
 // Bytes before the system table in the uploaded block (the BatchShape sits there).
 constexpr size_t kTableOffset = 256;
-// Points of a batched convolution work unit: 8 per thread of a 256-thread block.
-constexpr int64_t kConvPointsPerUnit = 8 * 256;
 // Atoms (sorted slots) of a batched gather work unit: four passes of a 256-thread block at
 // 5 atoms per warp.
 constexpr int64_t kGatherAtomsPerUnit = 4 * (256 / 32) * 5;
@@ -55,7 +61,7 @@ struct BatchLayout {
   int cap;
   size_t shape, sys, status, boxinfo, cl_sys, sup_sys, sidx, inv, pos, frac, bc, bh, sbc, sbh, nbr, ncount, itemoff, items;
   size_t lj, exslot, acc, e_tile;
-  size_t fix, real, cplx, partials, tickets, e_pme, pme_grad, pme_phi, moduli, twiddle;
+  size_t fix, real, cplx, partials, tickets, e_pme, pme_grad, pme_phi, moduli, tables;
   size_t bytes;
 };
 
@@ -107,7 +113,7 @@ inline BatchLayout batch_layout(int dtype, int64_t max_atoms, int64_t max_system
   L.pme_grad = take(3 * max_atoms * ts);
   L.pme_phi = take(max_atoms * ts);
   L.moduli = take((size_t)moduli_offset(kBatchMaxK + 1) * ts);
-  L.twiddle = take((size_t)twiddle_offset(kBatchMaxK + 1) * 2 * ts);
+  L.tables = take((size_t)table_offset(kBatchMaxK + 1) * 2 * ts);
   L.bytes = c.bytes();
   return L;
 }
@@ -117,13 +123,13 @@ inline BatchLayout batch_layout(int dtype, int64_t max_atoms, int64_t max_system
 
 using namespace tff;
 
-// Device pointers of one evaluation and the DFT size class: a captured graph replays only
+// Device pointers of one evaluation and the transform size class: a captured graph replays only
 // for the same key.
 struct BatchGraphKey {
   const void *ptr[10];
-  int dft_class;
+  int fft_class;
   bool operator==(const BatchGraphKey &o) const {
-    if (dft_class != o.dft_class) return false;
+    if (fft_class != o.fft_class) return false;
     for (int k = 0; k < 10; ++k)
       if (ptr[k] != o.ptr[k]) return false;
     return true;
@@ -168,14 +174,13 @@ void free_batch(tff_batch b) {
   delete b;
 }
 
-// DFT shared-memory size class of a batch, part of the graph key: 52 for grid sides up to
-// 52 (every water box up to 4,000 waters at 0.1 nm spacing), else the dtype's limit. A
-// class costs a capture per lane, and the shared memory of the class sets the resident DFT
-// blocks: 5 per SM at 52 (FP32), where a 56 class gave 4 (25 % slower passes) and 64 gave 3.
-constexpr int kDftSmallClass = 52;
-inline int dft_class(int kmax, int kcap) { return kmax <= kDftSmallClass ? std::min(kcap, kDftSmallClass) : kcap; }
+// Shared-memory size class of a batch's transforms, part of the graph key: 52 for grid sides up
+// to 52 (every water box up to 4,000 waters at 0.1 nm spacing), else the dtype's limit. A class
+// costs a capture per lane, and its shared memory (49 KB at 52 in FP32) sets the resident blocks.
+constexpr int kFftSmallClass = 52;
+inline int fft_class(int kmax, int kcap) { return kmax <= kFftSmallClass ? std::min(kcap, kFftSmallClass) : kcap; }
 
-// Host part of an evaluation: system table (offsets, cell grids, PME and DFT work units)
+// Host part of an evaluation: system table (offsets, cell grids, PME work units)
 // and shape into the pinned block, after the previous upload out of it is done. Returns
 // the table's largest grid side in *kmax.
 template <class T>
@@ -184,7 +189,7 @@ int batch_prepare(tff_batch b, int nsys, const int64_t *natoms, const int *pme_g
   auto &hs = b->host_sys;
   hs.assign(nsys, BatchSys{});
   int64_t ao = 0, co = 0, so = 0, go = 0, xo = 0;
-  int planes = 0, conv = 0, gat = 0;
+  int planes = 0, gat = 0;
   for (int i = 0; i < nsys; ++i) {
     const int64_t n = natoms[i];
     const int K = pme_grid[i];
@@ -202,17 +207,12 @@ int batch_prepare(tff_batch b, int nsys, const int64_t *natoms, const int *pme_g
     TFF_ARG((1 << (3 * y.bits)) <= kBatchMaxKeys, "system %d: cell grid too fine", i);
     y.K = K;
     y.mod_off = moduli_offset(K);
-    const int64_t ncplx = (int64_t)K * K * (K / 2 + 1);
+    y.table_off = table_offset(K);
     y.plane_off = planes;
-    // the convolution's units cover kConvPointsPerUnit points each (its PME blocks, sized
-    // for the atoms, mostly held a few points per thread at most)
-    y.conv_blocks = (int)std::min<int64_t>(kBatchPmeMaxBlocks, std::max<int64_t>(1, (ncplx + kConvPointsPerUnit - 1) / kConvPointsPerUnit));
-    y.conv_off = conv;
     // the gather's units take kGatherAtomsPerUnit atoms (the sorted slots of its clusters)
     y.gather_blocks = (int)std::min<int64_t>(kBatchPmeMaxBlocks, std::max<int64_t>(1, (y.ncl * kWarp + kGatherAtomsPerUnit - 1) / kGatherAtomsPerUnit));
     y.gather_off = gat;
     planes += K;
-    conv += y.conv_blocks;
     gat += y.gather_blocks;
     ao += n;
     co += y.ncl;
@@ -238,7 +238,6 @@ int batch_prepare(tff_batch b, int nsys, const int64_t *natoms, const int *pme_g
   sh.nsys = nsys;
   sh.plane_units = planes;
   sh.kmax = kmax;
-  sh.conv_units = conv;
   sh.gather_units = gat;
   // the pinned block is reused once the previous upload out of it is done
   TFF_CUDA(cudaEventSynchronize(b->table_ev));
@@ -249,7 +248,7 @@ int batch_prepare(tff_batch b, int nsys, const int64_t *natoms, const int *pme_g
 }
 
 // Device part of an evaluation on stream s (PME on the batch's second stream, joined back):
-// every launch shape depends on the batch's capacity and the DFT class alone, so the
+// every launch shape depends on the batch's capacity and the transform class alone, so the
 // sequence can be captured once and replayed for any composition of that class.
 template <class T>
 int batch_enqueue(tff_batch b, int kclass, const T *x, const T *boxes, const T *q, const T *sigma, const T *eps,
@@ -309,35 +308,19 @@ int batch_enqueue(tff_batch b, int kclass, const T *x, const T *boxes, const T *
   unsigned *counters = cd.status + 16;
   batch_spread_kernel<T><<<nb_pme, kPmeBlock, 0, ps>>>(dsys, shape, x, q, boxes, fix, counters);
   TFF_LAUNCHED();
-  T *real;
-  if (sizeof(T) == 4) {
-    real = reinterpret_cast<T *>(w + L.real);
-    batch_fix_to_real_kernel<<<sms * 8, 256, 0, ps>>>(shape, reinterpret_cast<unsigned long long *>(fix),
-                                                     reinterpret_cast<float *>(real));
-    TFF_LAUNCHED();
-  } else {
-    real = reinterpret_cast<T *>(fix);
-  }
-  auto *cplx = reinterpret_cast<typename CplxOf<T>::type *>(w + L.cplx);
-  const auto *twtab = reinterpret_cast<const typename CplxOf<T>::type *>(w + L.twiddle);
-  const size_t dsmem = batch_dft_smem<T>(kclass);
-  const int nb_dft = sms * 8;
-  batch_dft_kernel<T, kDftZR2C><<<nb_dft, kDftThreads, dsmem, ps>>>(dsys, shape, real, cplx, twtab, counters + 1);
-  TFF_LAUNCHED();
-  batch_dft_kernel<T, kDftY><<<nb_dft, kDftThreads, dsmem, ps>>>(dsys, shape, real, cplx, twtab, counters + 2);
-  TFF_LAUNCHED();
-  batch_dft_kernel<T, kDftX><<<nb_dft, kDftThreads, dsmem, ps>>>(dsys, shape, real, cplx, twtab, counters + 3);
-  TFF_LAUNCHED();
-  batch_convolve_kernel<T><<<nb_pme, kPmeBlock, 0, ps>>>(dsys, shape, cplx, boxes, b->desc.ewald_alpha,
-                                                         reinterpret_cast<const T *>(w + L.moduli), partials, tickets,
-                                                         e_pme, counters + 4);
-  TFF_LAUNCHED();
-  batch_dft_kernel<T, kDftXInv><<<nb_dft, kDftThreads, dsmem, ps>>>(dsys, shape, real, cplx, twtab, counters + 5);
-  TFF_LAUNCHED();
-  batch_dft_kernel<T, kDftYInv><<<nb_dft, kDftThreads, dsmem, ps>>>(dsys, shape, real, cplx, twtab, counters + 6);
-  TFF_LAUNCHED();
-  batch_dft_kernel<T, kDftZC2R><<<nb_dft, kDftThreads, dsmem, ps>>>(dsys, shape, real, cplx, twtab, counters + 7);
-  TFF_LAUNCHED();
+  T *real = sizeof(T) == 4 ? reinterpret_cast<T *>(w + L.real) : reinterpret_cast<T *>(fix);
+  auto *cplx = reinterpret_cast<Cplx<T> *>(w + L.cplx);
+  const auto *tables = reinterpret_cast<const Cplx<T> *>(w + L.tables);
+  const T *moduli = reinterpret_cast<const T *>(w + L.moduli);
+  const size_t fsmem = fft_smem<T>(kclass);
+  const auto fft = [&](auto kernel, unsigned *counter) {
+    kernel<<<sms * 4, kBatchFftThreads, fsmem, ps>>>(dsys, shape, fix, real, cplx, tables, boxes, b->desc.ewald_alpha,
+                                                     moduli, partials, tickets, e_pme, counter);
+    return cudaGetLastError();
+  };
+  TFF_CUDA(fft(batch_fft_kernel<T, kFftForward>, counters + 1));
+  TFF_CUDA(fft(batch_fft_kernel<T, kFftSolve>, counters + 2));
+  TFF_CUDA(fft(batch_fft_kernel<T, kFftInverse>, counters + 3));
 
   // --- real space on the caller stream
   S *gx = reinterpret_cast<S *>(w + L.acc);
@@ -349,7 +332,7 @@ int batch_enqueue(tff_batch b, int kclass, const T *x, const T *boxes, const T *
   TFF_CUDA(cudaEventRecord(b->sorted_ev, s));
   TFF_CUDA(cudaStreamWaitEvent(ps, b->sorted_ev, 0));
   batch_gather_kernel<T><<<nb_pme, kPmeBlock, 0, ps>>>(dsys, shape, x, q, cd.sidx, boxes, real, b->desc.ewald_alpha,
-                                                       pme_phi, pme_grad, partials, tickets, e_pme, counters + 8);
+                                                       pme_phi, pme_grad, partials, tickets, e_pme, counters + 4);
   TFF_LAUNCHED();
   TFF_CUDA(cudaEventRecord(b->join_ev, ps));
   cluster_bounds_kernel<T><<<(int)std::max<int64_t>(1, std::min<int64_t>(L.supers, 2 * sms)), kWarp * kSuper, 0, s>>>(cd);
@@ -389,7 +372,7 @@ int batch_enqueue(tff_batch b, int kclass, const T *x, const T *boxes, const T *
   return TFF_OK;
 }
 
-// Most graphs a batch keeps (one per DFT class and buffer set; the oldest goes first).
+// Most graphs a batch keeps (one per transform class and buffer set; the oldest goes first).
 constexpr size_t kBatchMaxGraphs = 8;
 
 // Captures the device part for `key` (nothing runs) and appends the graph to the batch's
@@ -399,7 +382,7 @@ int batch_capture(tff_batch b, const BatchGraphKey &key, const T *x, const T *bo
                   const T *eps, const int *excl, double *energies, T *forces) {
   if (b->capture_stream == nullptr) TFF_CUDA(cudaStreamCreateWithFlags(&b->capture_stream, cudaStreamNonBlocking));
   TFF_CUDA(cudaStreamBeginCapture(b->capture_stream, cudaStreamCaptureModeThreadLocal));
-  const int st = batch_enqueue<T>(b, key.dft_class, x, boxes, q, sigma, eps, excl, energies, forces,
+  const int st = batch_enqueue<T>(b, key.fft_class, x, boxes, q, sigma, eps, excl, energies, forces,
                                   b->capture_stream);
   cudaGraph_t graph = nullptr;
   const cudaError_t ee = cudaStreamEndCapture(b->capture_stream, &graph);
@@ -427,7 +410,7 @@ int batch_eval_impl(tff_batch b, int nsys, const int64_t *natoms, const int *pme
   int kmax = 6;
   int st = batch_prepare<T>(b, nsys, natoms, pme_grid, &kmax);
   if (st != TFF_OK) return st;
-  const int kclass = dft_class(kmax, sizeof(T) == 8 ? kBatchMaxK64 : kBatchMaxK);
+  const int kclass = fft_class(kmax, sizeof(T) == 8 ? kBatchMaxK64 : kBatchMaxK);
   // upload the shape and the table (exact size), then run the device part
   TFF_CUDA(cudaMemcpyAsync(b->ws + b->L.shape, b->table, kTableOffset + nsys * sizeof(BatchSys),
                            cudaMemcpyHostToDevice, s));
@@ -453,26 +436,23 @@ template <class T>
 int set_sort_smem() {
   TFF_CUDA(cudaFuncSetAttribute(batch_sort_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)kBatchSortSmem));
-  const int dft = (int)batch_dft_smem<T>(sizeof(T) == 8 ? kBatchMaxK64 : kBatchMaxK);
-  TFF_CUDA(cudaFuncSetAttribute(batch_dft_kernel<T, kDftZR2C>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft));
-  TFF_CUDA(cudaFuncSetAttribute(batch_dft_kernel<T, kDftY>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft));
-  TFF_CUDA(cudaFuncSetAttribute(batch_dft_kernel<T, kDftX>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft));
-  TFF_CUDA(cudaFuncSetAttribute(batch_dft_kernel<T, kDftXInv>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft));
-  TFF_CUDA(cudaFuncSetAttribute(batch_dft_kernel<T, kDftYInv>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft));
-  TFF_CUDA(cudaFuncSetAttribute(batch_dft_kernel<T, kDftZC2R>, cudaFuncAttributeMaxDynamicSharedMemorySize, dft));
+  const int smem = (int)fft_smem<T>(sizeof(T) == 8 ? kBatchMaxK64 : kBatchMaxK);
+  TFF_CUDA(cudaFuncSetAttribute(batch_fft_kernel<T, kFftForward>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  TFF_CUDA(cudaFuncSetAttribute(batch_fft_kernel<T, kFftSolve>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  TFF_CUDA(cudaFuncSetAttribute(batch_fft_kernel<T, kFftInverse>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   return TFF_OK;
 }
 
 }  // namespace
 
-// Captures the graph of the batch's common DFT class (grid sides up to 52) for these
+// Captures the graph of the batch's common transform class (grid sides up to 52) for these
 // device buffers ahead of use, so that the first evaluations through them need no capture
 // (used for the server's lanes, whose staging buffers never change).
 int batch_warm_graph(tff_batch b, const void *coords, const void *boxes, const void *charges, const void *sigma,
                      const void *epsilon, const int *excl, double *energies, void *forces) {
   const int kcap = b->desc.dtype == TFF_F64 ? kBatchMaxK64 : kBatchMaxK;
   const BatchGraphKey key{{coords, boxes, charges, sigma, epsilon, excl, energies, forces, nullptr, nullptr},
-                          dft_class(6, kcap)};
+                          fft_class(6, kcap)};
   if (b->desc.dtype == TFF_F32)
     return batch_capture<float>(b, key, (const float *)coords, (const float *)boxes, (const float *)charges,
                                 (const float *)sigma, (const float *)epsilon, excl, energies, (float *)forces);
@@ -531,14 +511,13 @@ int tff_batch_create(const tff_batch_desc *desc, tff_batch *out) {
     }
   }
   if (e == cudaSuccess) {
-    // twiddles of every grid side the batch accepts (the DFT passes read them per plane)
-    if (desc->dtype == TFF_F64)
-      batch_twiddle_kernel<double><<<64, 256>>>(reinterpret_cast<CplxOf<double>::type *>(b->ws + b->L.twiddle),
-                                                kBatchMaxK);
-    else
-      batch_twiddle_kernel<float><<<64, 256>>>(reinterpret_cast<CplxOf<float>::type *>(b->ws + b->L.twiddle),
-                                               kBatchMaxK);
-    e = cudaGetLastError();
+    // transform tables of every grid side the batch accepts
+    const auto upload = [&](auto zero) {
+      std::vector<Cplx<decltype(zero)>> tab;
+      for (int K = 6; K <= kBatchMaxK; ++K) fft_table(K, tab);
+      return cudaMemcpy(b->ws + b->L.tables, tab.data(), tab.size() * sizeof(tab[0]), cudaMemcpyHostToDevice);
+    };
+    e = desc->dtype == TFF_F64 ? upload(0.0) : upload(0.0f);
     if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);  // the PME streams do not wait for stream 0
   }
   if (e != cudaSuccess) {
@@ -591,8 +570,8 @@ int64_t tff_batch_graph_launches(tff_batch b) { return b ? b->graph_launches : 0
 int tff_batch_kernel_launches(tff_batch b) {
   if (!b) return 0;
   // sort, bounds, neighbours, params, pair kernel, finalize; grid zeroing, spread,
-  // [to_real], 3 DFT passes, convolve, 3 inverse passes, gather
-  return 6 + (b->desc.dtype == TFF_F32 ? 11 : 10);
+  // three transform passes, gather
+  return 6 + 6;
 }
 
 }  // extern "C"

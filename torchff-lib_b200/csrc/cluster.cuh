@@ -133,12 +133,10 @@ struct BatchSys {
   int64_t grid_off, cplx_off;  // PME grids: K^3 real points, K*K*(K/2+1) complex points
   int nc, bits;                // cell grid side and Hilbert bits per axis
   int K, mod_off;              // PME grid side and offset of its B-spline moduli
-  int plane_off;               // the system's first DFT plane unit (sum of K before it)
-  int conv_blocks;             // work units (and reduction blocks) of its convolution
-  int conv_off;                // the system's first convolution unit (sum of conv_blocks before it)
+  int plane_off;               // the system's first transform plane (sum of K before it)
   int gather_blocks;           // work units (and reduction blocks) of its force gather; the spread's too
   int gather_off;              // the system's first gather unit
-  int pad;
+  int table_off;               // its grid side's transform tables
 };
 
 // Totals of a batch, in device memory beside its system table: the batched kernels read
@@ -147,9 +145,8 @@ struct BatchSys {
 struct BatchShape {
   int64_t natoms, nclusters, npad, nsuper, total_grid;
   int nsys;
-  int plane_units;  // DFT plane units: sum of K
+  int plane_units;  // transform planes: sum of K
   int kmax;
-  int conv_units;   // convolution units: sum of conv_blocks
   int gather_units; // gather (and spread) units: sum of gather_blocks
   int pad;
 };

@@ -791,10 +791,10 @@ int tff_system_hvp(tff_system sys, const void *coords, const void *box, const vo
 
 int tff_system_kernel_launches(tff_system sys) {
   if (!sys) return 0;
-  // cluster build 7 (1 for a small system) + sorted params 1 + tile 1 + finalize 1; PME: spread,
-  // [to_real], convolve, gather
+  // cluster build 7 (1 for a small system) + sorted params 1 + tile 1 + finalize 1; PME: spread, solve,
+  // gather. The solve is three plane kernels, or [to_real] and the convolution between cuFFT's
   int k = small_build(sys->cl) ? 4 : 10;
-  if (sys->pme) k += sys->desc.dtype == TFF_F32 ? 4 : 3;
+  if (sys->pme) k += sys->pme->impl.planes ? 5 : sys->desc.dtype == TFF_F32 ? 4 : 3;
   return k;
 }
 

@@ -1,10 +1,11 @@
 // Rank-0 smooth PME (order-6 B-splines) on a cubic K^3 grid.
 //
 //   spread   : Q(g) = sum_i q_i M6(u_i,x) M6(u_i,y) M6(u_i,z)   (fixed-point or FP64 atomics)
-//   [to_real]: fixed-point grid -> FP32 (mixed precision)
-//   R2C FFT  : S(k)                                             (cuFFT)
+//   R2C FFT  : S(k)
 //   convolve : S(k) *= C(k)/theta(k)^2, E_rec = 1/2 sum_k C |S|^2/theta^2 (FP64, fixed order)
-//   C2R FFT  : Phi(g)                                           (cuFFT, unnormalised)
+//   C2R FFT  : Phi(g)                                           (unnormalised)
+//              these three by the plane kernels of pme_fft.cuh, or by cuFFT for the grid sides it
+//              takes less time for (fft_planes)
 //   gather   : phi_i = sum_g theta_i(g) Phi(g), dE/dx_i = q_i grad phi_i,
 //              dE/dq_i = phi_i - 2 a q_i / sqrt(pi), E_self = -(a/sqrt(pi)) sum q^2
 //
@@ -16,9 +17,8 @@
 
 #include <cufft.h>
 
-#include <type_traits>
-
 #include "cluster.cuh"
+#include "pme_fft.cuh"
 
 namespace tff {
 
@@ -40,7 +40,7 @@ __device__ __forceinline__ void load_pme_shared(const T *box, int K, PmeShared &
   sh.vol = b.vol;
 }
 
-// Atom sources: plain (caller arrays) or cluster-sorted (wrapped positions, charge in .w).
+// Atom sources: caller order, or caller arrays in the order of a cluster build.
 template <class T>
 struct PlainAtoms {
   const T *x;
@@ -50,20 +50,6 @@ struct PlainAtoms {
     if (t >= n) return false;
     rx = x[3 * t]; ry = x[3 * t + 1]; rz = x[3 * t + 2];
     qi = q[t];
-    return true;
-  }
-};
-
-template <class T>
-struct SortedAtoms {
-  const typename V4<T>::type *pos;
-  const int *sidx;
-  int64_t npad;
-  __device__ __forceinline__ bool get(int64_t t, double &rx, double &ry, double &rz, T &qi) const {
-    if (t >= npad || sidx[t] < 0) return false;
-    const auto p = pos[t];
-    rx = p.x; ry = p.y; rz = p.z;
-    qi = p.w;
     return true;
   }
 };
@@ -215,79 +201,40 @@ __global__ void __launch_bounds__(kPmeBlock) pme_spread_kernel(Atoms atoms, int6
 // Blocks of a kernel that takes one atom (spread) or kGatherAtomsPerWarp (gather) per warp at a
 // time, up to a few waves.
 inline int pme_blocks(int64_t warps) {
-  return (int)std::max<int64_t>(1, std::min<int64_t>((warps * kWarp + kPmeBlock - 1) / kPmeBlock, (int64_t)sm_count() * 8));
-}
-
-static __global__ void pme_fix_to_real_kernel(const unsigned long long *gi, float *gf, int64_t n) {
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-    gf[k] = (float)from_fix(gi[k]);
+  const int64_t blocks = (warps * kWarp + kPmeBlock - 1) / kPmeBlock;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)sm_count() * 8));
 }
 
 template <class T> struct CplxOf;
 template <> struct CplxOf<float> { using type = cufftComplex; };
 template <> struct CplxOf<double> { using type = cufftDoubleComplex; };
 
-// Convolution of the points bid, bid + nblk, ... (in blocks of blockDim.x); returns this
-// thread's share of sum_k w C(k) |S(k)|^2 / theta(k)^2 (the energy is half of the total).
-template <class T>
-__device__ __forceinline__ double convolve_points(typename CplxOf<T>::type *S, const PmeShared &sh, int K,
-                                                  double alpha, const T *xmod, const T *ymod, const T *zmod,
-                                                  int64_t bid, int64_t nblk) {
-  const int Kz = K / 2 + 1;
-  const int64_t total = (int64_t)K * K * Kz;
-  const double four_pi_over_v = 4.0 * 3.14159265358979323846 / sh.vol;
-  const double two_pi = 2.0 * 3.14159265358979323846;
-  const double inv4a2 = 1.0 / (4.0 * alpha * alpha);
-  double e = 0.0;
-  // 32-bit index arithmetic (a 64-bit division costs several times a 32-bit one) while the
-  // grid has fewer than 2^32 points, i.e. for every K below 2048
-  const bool narrow = total < (int64_t(1) << 32);
-  for (int64_t t = bid * blockDim.x + threadIdx.x; t < total; t += nblk * blockDim.x) {
-    int ix, iy, iz;
-    if (narrow) {
-      const unsigned tt = (unsigned)t, row = tt / (unsigned)Kz, x = row / (unsigned)K;
-      iz = (int)(tt - row * (unsigned)Kz);
-      iy = (int)(row - x * (unsigned)K);
-      ix = (int)x;
-    } else {
-      iz = (int)(t % Kz);
-      iy = (int)((t / Kz) % K);
-      ix = (int)(t / ((int64_t)Kz * K));
-    }
-    const double mx = (2 * ix < K) ? ix : ix - K;
-    const double my = (2 * iy < K) ? iy : iy - K;
-    const double mz = (2 * iz < K) ? iz : iz - K;
-    double factor = 0.0;
-    if (t != 0) {
-      // k_c = 2 pi sum_d m_d inv[c][d]
-      const double kx = two_pi * (mx * sh.inv[0] + my * sh.inv[1] + mz * sh.inv[2]);
-      const double ky = two_pi * (mx * sh.inv[3] + my * sh.inv[4] + mz * sh.inv[5]);
-      const double kz = two_pi * (mx * sh.inv[6] + my * sh.inv[7] + mz * sh.inv[8]);
-      const double ksq = kx * kx + ky * ky + kz * kz;
-      const double th = (double)xmod[ix] * (double)ymod[iy] * (double)zmod[iz];
-      factor = four_pi_over_v * exp(-ksq * inv4a2) / (ksq * th * th);
-    }
-    auto v = S[t];
-    const double re = v.x, im = v.y;
-    const double w = (iz == 0 || 2 * iz == K) ? 1.0 : 2.0;
-    e += w * factor * (re * re + im * im);
-    v.x = (T)(re * factor);
-    v.y = (T)(im * factor);
-    S[t] = v;
-  }
-  return e;
+// Influence function C(k) / theta(k)^2 of a box, C(k) = 4 pi exp(-k^2 / 4 alpha^2) / (V k^2).
+struct Influence {
+  double inv[9], four_pi_over_v, inv4a2;
+};
+
+__device__ __forceinline__ void load_influence(const PmeShared &sh, double alpha, Influence &f) {
+  for (int k = 0; k < 9; ++k) f.inv[k] = sh.inv[k];
+  f.four_pi_over_v = 4.0 * 3.14159265358979323846 / sh.vol;
+  f.inv4a2 = 1.0 / (4.0 * alpha * alpha);
 }
 
 template <class T>
-__global__ void __launch_bounds__(kPmeBlock) pme_convolve_kernel(typename CplxOf<T>::type *S, const T *box, int K,
-                                                                 double alpha, const T *xmod, const T *ymod,
-                                                                 const T *zmod, double *partials, unsigned *ticket,
-                                                                 double *e_rec) {
-  __shared__ PmeShared sh;
-  if (threadIdx.x == 0) load_pme_shared(box, K, sh);
-  __syncthreads();
-  const double e = convolve_points<T>(S, sh, K, alpha, xmod, ymod, zmod, blockIdx.x, gridDim.x);
-  grid_sum<kPmeBlock>(0.5 * e, partials, ticket, e_rec, false);
+__device__ __forceinline__ double influence(const Influence &f, int K, int ix, int iy, int iz, const T *xmod,
+                                            const T *ymod, const T *zmod) {
+  if (ix == 0 && iy == 0 && iz == 0) return 0.0;
+  const double two_pi = 2.0 * 3.14159265358979323846;
+  const double mx = (2 * ix < K) ? ix : ix - K;
+  const double my = (2 * iy < K) ? iy : iy - K;
+  const double mz = (2 * iz < K) ? iz : iz - K;
+  // k_c = 2 pi sum_d m_d inv[c][d]
+  const double kx = two_pi * (mx * f.inv[0] + my * f.inv[1] + mz * f.inv[2]);
+  const double ky = two_pi * (mx * f.inv[3] + my * f.inv[4] + mz * f.inv[5]);
+  const double kz = two_pi * (mx * f.inv[6] + my * f.inv[7] + mz * f.inv[8]);
+  const double ksq = kx * kx + ky * ky + kz * kz;
+  const double th = (double)xmod[ix] * (double)ymod[iy] * (double)zmod[iz];
+  return f.four_pi_over_v * exp(-ksq * f.inv4a2) / (ksq * th * th);
 }
 
 // Gather output: caller arrays (caller order), plain stores (one thread per atom).
@@ -610,27 +557,10 @@ __global__ void __launch_bounds__(kPmeBlock) pme_gather_hvp_kernel(PlainAtoms<T>
   }
 }
 
-// ---- batched 3-D real DFT of many grids of different sizes (the serving path)
-// One launch per axis pass over every system of a batch. The work units are the planes of
-// every grid (system s owns units plane_off .. plane_off + K - 1); blocks loop over them.
-// A block stages one plane in shared memory as `lines` x `points` with an
-// odd row stride (so lanes reading one point of consecutive lines hit distinct banks),
-// evaluates each output as a direct sum over the line with a twiddle table
-// w[m] = exp(-+2 pi i m / K) (consecutive lanes share the twiddle: a broadcast), stages
-// the outputs and writes them back contiguously. Layouts are those of cuFFT's R2C/C2R:
-// real grid [x][y][z] (K^3), half spectrum [kx][ky][kz] (K x K x (K/2+1)), the inverse
-// unnormalised. The summation order is fixed, so a grid's result does not depend on the
-// batch it runs in.
-enum BatchDftPass { kDftZR2C = 0, kDftY, kDftX, kDftXInv, kDftYInv, kDftZC2R };
-constexpr int kDftThreads = 256;
-
-__host__ __device__ inline int dft_stride(int K) { return K | 1; }
-
-// Shared memory of one block of a pass for grid side K (twiddles + input + output planes).
-template <class T>
-inline size_t batch_dft_smem(int K) {
-  return (size_t)(K + 2 * (size_t)K * dft_stride(K)) * 2 * sizeof(T);
-}
+// ---- batched transforms: the plane kernels of pme_fft.cuh over every system of a batch. The work
+// units are the planes of every grid (system s owns units plane_off .. plane_off + K - 1); the
+// summation order of a plane is fixed, so a grid's result does not depend on the batch it runs in.
+constexpr int kBatchFftThreads = 256;
 
 // Next work unit of a persistent batched kernel, drawn from a per-launch counter (zeroed
 // before the launch) so that blocks that finish early take more: returns the unit, equal
@@ -645,17 +575,15 @@ __device__ __forceinline__ int next_unit(unsigned *counter) {
 }
 
 // The batch system owning work unit u: the largest s < nsys whose first unit (plane_off for
-// DFT planes, conv_off for convolution units, gather_off for gather and spread units) is at
+// transform planes, gather_off for gather and spread units) is at
 // most u. Every system owns at least one unit of each kind.
-enum BatchUnits { kUnitsPlanes = 0, kUnitsConv, kUnitsGather };
+enum BatchUnits { kUnitsPlanes = 0, kUnitsGather };
 template <int KIND>
 __device__ __forceinline__ int unit_system(const BatchSys *sys, int nsys, int u) {
   int lo = 0, hi = nsys - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    const int off = KIND == kUnitsPlanes ? sys[mid].plane_off
-                    : KIND == kUnitsConv ? sys[mid].conv_off
-                                         : sys[mid].gather_off;
+    const int off = KIND == kUnitsPlanes ? sys[mid].plane_off : sys[mid].gather_off;
     if (off <= u)
       lo = mid;
     else
@@ -664,190 +592,63 @@ __device__ __forceinline__ int unit_system(const BatchSys *sys, int nsys, int u)
   return lo;
 }
 
-// Twiddle table of every grid side 1..kmax: side K at offset K (K - 1) / 2 holds
-// exp(-2 pi i m / K), m = 0..K-1, rounded from FP64. Filled once per batch object.
-__host__ __device__ inline int64_t twiddle_offset(int K) { return (int64_t)K * (K - 1) / 2; }
-
-template <class T>
-__global__ void batch_twiddle_kernel(typename CplxOf<T>::type *tab, int kmax) {
-  const int64_t n = twiddle_offset(kmax + 1);
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    int K = (int)((1.0 + sqrt(1.0 + 8.0 * (double)e)) / 2.0);  // twiddle_offset(K) <= e < twiddle_offset(K + 1)
-    while (twiddle_offset(K) > e) --K;
-    while (twiddle_offset(K + 1) <= e) ++K;
-    const int m = (int)(e - twiddle_offset(K));
-    double sn, cs;
-    sincospi(2.0 * m / K, &sn, &cs);
-    tab[e].x = (T)cs;
-    tab[e].y = (T)(-sn);
-  }
-}
-
-// Lines of a plane each thread transforms at once (one twiddle load serves them all).
-// Measured on a 256-system serving batch (0.85 M atoms): 1 -> 2 -> 4 lines per thread
-// 4.37 -> 4.27 -> 4.25 ms, 8 lines 4.38 ms.
-constexpr int kDftLinesPerThread = 4;
-
-// One plane p of one grid (see batch_dft_kernel); twtab: the batch's twiddle table.
-template <class T, int PASS>
-__device__ __forceinline__ void batch_dft_plane(const BatchSys &b, const int p, T *real, typename CplxOf<T>::type *cplx,
-                                                const typename CplxOf<T>::type *twtab) {
-  using C = typename CplxOf<T>::type;
-  const int K = b.K;
-  const int Kz = K / 2 + 1, st = dft_stride(K);
-  constexpr bool kInverse = PASS >= kDftXInv;
-  extern __shared__ __align__(16) unsigned char dft_smem[];
-  C *tw = reinterpret_cast<C *>(dft_smem);
-  C *in = tw + K;
-  C *out = in + (size_t)K * st;
-  for (int m = threadIdx.x; m < K; m += blockDim.x) {
-    C v = twtab[twiddle_offset(K) + m];
-    if (kInverse) v.y = -v.y;
-    tw[m] = v;
-  }
-  // plane geometry: lines x points in, lines x nout out
-  const int lines = (PASS == kDftZR2C || PASS == kDftZC2R) ? K : Kz;
-  const int points = PASS == kDftZC2R ? Kz : K;
-  const int nout = PASS == kDftZR2C ? Kz : K;
-  T *rgrid = real + b.grid_off;
-  C *cgrid = cplx + b.cplx_off;
-  // load (global-contiguous order)
-  for (int e = threadIdx.x; e < lines * points; e += blockDim.x) {
-    int line, pt;
-    C v;
-    if (PASS == kDftZR2C) {  // plane x: [y][z] reals
-      line = e / K;
-      pt = e % K;
-      v.x = rgrid[(int64_t)p * K * K + e];
-      v.y = T(0);
-    } else if (PASS == kDftZC2R) {  // plane x: [y][kz]
-      line = e / Kz;
-      pt = e % Kz;
-      v = cgrid[(int64_t)p * K * Kz + e];
-    } else if (PASS == kDftY || PASS == kDftYInv) {  // plane x: [y][kz], lines = kz
-      pt = e / Kz;
-      line = e % Kz;
-      v = cgrid[(int64_t)p * K * Kz + e];
-    } else {  // plane ky: [x][ky][kz], lines = kz
-      pt = e / Kz;
-      line = e % Kz;
-      v = cgrid[((int64_t)pt * K + p) * Kz + line];
-    }
-    in[line * st + pt] = v;
-  }
-  __syncthreads();
-  // outputs: one frequency (or z) per thread for R lines lg, lg + G, ... (G = ceil(lines / R)):
-  // consecutive lanes take consecutive lines (odd row stride: distinct banks) and each
-  // twiddle load serves R lines. Per output the sum runs over the line in a fixed order.
-  constexpr int R = kDftLinesPerThread;
-  const int G = (lines + R - 1) / R;
-  for (int o = threadIdx.x; o < G * nout; o += blockDim.x) {
-    const int lg = o % G, f = o / G;
-    bool has[R];
-    const C *row[R];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      has[r] = lg + r * G < lines;
-      row[r] = in + (has[r] ? lg + r * G : lg) * st;
-    }
-    C acc[R];
-    if (PASS == kDftZC2R) {
-      // real output of a Hermitian half spectrum: T0 + 2 sum_{0<k<K/2} Re(Tk w^(zk)) [+ T_{K/2} (-1)^z]
-      const int kh = (K - 1) / 2;
-      T sum[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) sum[r] = row[r][0].x;
-      int idx = 0;
-      for (int k = 1; k <= kh; ++k) {
-        idx += f;
-        if (idx >= K) idx -= K;
-        const C w = tw[idx];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const C a = row[r][k];
-          sum[r] += T(2) * (a.x * w.x - a.y * w.y);
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (!(K & 1)) sum[r] += (f & 1) ? -row[r][K / 2].x : row[r][K / 2].x;
-        acc[r].x = sum[r];
-        acc[r].y = T(0);
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < R; ++r) acc[r].x = acc[r].y = T(0);
-      int idx = 0;
-      for (int j = 0; j < points; ++j) {
-        const C w = tw[idx];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          const C a = row[r][j];
-          if (PASS == kDftZR2C) {  // real input
-            acc[r].x += a.x * w.x;
-            acc[r].y += a.x * w.y;
-          } else {
-            acc[r].x += a.x * w.x - a.y * w.y;
-            acc[r].y += a.x * w.y + a.y * w.x;
-          }
-        }
-        idx += f;
-        if (idx >= K) idx -= K;
-      }
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (has[r]) out[(lg + r * G) * st + f] = acc[r];
-  }
-  __syncthreads();
-  // store (global-contiguous order)
-  for (int e = threadIdx.x; e < lines * nout; e += blockDim.x) {
-    if (PASS == kDftZR2C) {  // [y][kz]
-      cgrid[(int64_t)p * K * Kz + e] = out[(e / Kz) * st + e % Kz];
-    } else if (PASS == kDftZC2R) {  // [y][z] reals
-      rgrid[(int64_t)p * K * K + e] = out[(e / K) * st + e % K].x;
-    } else if (PASS == kDftY || PASS == kDftYInv) {  // [ky][kz], lines = kz
-      cgrid[(int64_t)p * K * Kz + e] = out[(e % Kz) * st + e / Kz];
-    } else {  // [kx][ky][kz], lines = kz
-      const int f = e / Kz, line = e % Kz;
-      cgrid[((int64_t)f * K + p) * Kz + line] = out[line * st + f];
-    }
-  }
-}
-
-template <class T, int PASS>
-__global__ void __launch_bounds__(kDftThreads) batch_dft_kernel(const BatchSys *sys, const BatchShape *shape, T *real,
-                                                                typename CplxOf<T>::type *cplx,
-                                                                const typename CplxOf<T>::type *twtab,
-                                                                unsigned *counter) {
-  const int nsys = shape->nsys, units = shape->plane_units;
-  for (int u = next_unit(counter); u < units; u = next_unit(counter)) {
-    const BatchSys &b = sys[unit_system<kUnitsPlanes>(sys, nsys, u)];
-    batch_dft_plane<T, PASS>(b, u - b.plane_off, real, cplx, twtab);
-  }
-}
-
-// ---- batched PME: persistent kernels over work units numbered across the batch. The spread
-// and the gather take units of a system's atoms (system s owns gather_off .. gather_off +
-// gather_blocks - 1), the convolution units of its grid points (conv_off ..); a unit count
-// depends on the system alone, so that its reductions sum in the same order whatever else
-// is in the batch. The spread and the convolution keep 4 resident blocks per SM (at most 64
-// registers): the loop's extra state had cost them a block per SM and 29 % / 67 % of their
-// time at 256 systems.
+// Persistent kernels over work units numbered across the batch: the planes of every grid, and
+// units of a system's atoms for the spread and the gather (system s owns gather_off .. gather_off +
+// gather_blocks - 1). A unit count depends on the system alone, so that its reductions sum in the
+// same order whatever else is in the batch. Most blocks of a system's reductions:
 constexpr int kBatchPmeMaxBlocks = 256;
 
-// Zeroes the batch's accumulation grid (total_grid points of the shape).
+enum BatchFftPass { kFftForward = 0, kFftSolve, kFftInverse };
+
+template <class T, int PASS>
+__device__ __forceinline__ void batch_fft_unit(const BatchSys &b, int sy, int p, typename Acc<T>::S *grid, T *real,
+                                               Cplx<T> *cplx, const Cplx<T> *tables, const T *boxes, double alpha,
+                                               const T *moduli, double *partials, unsigned *tickets, double *energies,
+                                               PmeShared &sh, Influence &inf) {
+  const int K = b.K, Kz = K / 2 + 1;
+  FftPlan f = fft_plan<T>(K, tables + b.table_off);
+  Cplx<T> *spec = cplx + b.cplx_off;
+  const auto nothing = [] {};
+  if constexpr (PASS == kFftForward) {
+    fft_forward_plane<T>(f, grid + b.grid_off + (int64_t)p * K * K, spec + (int64_t)p * K * Kz, nothing);
+  } else if constexpr (PASS == kFftInverse) {
+    fft_inverse_plane<T>(f, spec + (int64_t)p * K * Kz, real + b.grid_off + (int64_t)p * K * K, nothing);
+  } else {
+    if (threadIdx.x == 0) {
+      load_pme_shared(boxes + 9 * (int64_t)sy, K, sh);
+      load_influence(sh, alpha, inf);
+    }
+    __syncthreads();
+    const T *xm = moduli + b.mod_off, *ym = xm + K, *zm = ym + K;
+    const double e = fft_solve_row<T>(
+        f, spec, p, 0, Kz, [&](int ix, int iz) { return influence<T>(inf, K, ix, p, iz, xm, ym, zm); }, nothing, nothing);
+    grid_sum_n<kBatchFftThreads>(0.5 * e, partials + (int64_t)kBatchPmeMaxBlocks * sy, tickets + 2 * sy,
+                                 energies + 2 * sy, false, p, K);
+  }
+}
+
+// partials: kBatchPmeMaxBlocks per system; tickets and energies: 2 per system
+// ([2s] reciprocal, [2s+1] self).
+template <class T, int PASS>
+__global__ void __launch_bounds__(kBatchFftThreads, sizeof(T) == 4 ? 3 : 2)
+    batch_fft_kernel(const BatchSys *sys, const BatchShape *shape, typename Acc<T>::S *grid, T *real, Cplx<T> *cplx,
+                     const Cplx<T> *tables, const T *boxes, double alpha, const T *moduli, double *partials,
+                     unsigned *tickets, double *energies, unsigned *counter) {
+  __shared__ PmeShared sh;
+  __shared__ Influence inf;
+  const int nsys = shape->nsys, units = shape->plane_units;
+  for (int u = next_unit(counter); u < units; u = next_unit(counter)) {
+    const int sy = unit_system<kUnitsPlanes>(sys, nsys, u);
+    batch_fft_unit<T, PASS>(sys[sy], sy, u - sys[sy].plane_off, grid, real, cplx, tables, boxes, alpha, moduli, partials,
+                            tickets, energies, sh, inf);
+  }
+}
+
 template <class S>
 __global__ void batch_zero_grid_kernel(const BatchShape *shape, S *grid) {
   const int64_t n = shape->total_grid;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-    grid[k] = S(0);
-}
-
-static __global__ void batch_fix_to_real_kernel(const BatchShape *shape, const unsigned long long *gi, float *gf) {
-  const int64_t n = shape->total_grid;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-    gf[k] = (float)from_fix(gi[k]);
+    grid[k] = 0;
 }
 
 // One PME block of one system (a separate call: the unit loop's state then does not share
@@ -874,29 +675,6 @@ __global__ void __launch_bounds__(kPmeBlock, 4) batch_spread_kernel(const BatchS
   for (int u = next_unit(counter); u < units; u = next_unit(counter)) {
     const int sy = unit_system<kUnitsGather>(sys, nsys, u);
     batch_spread_unit<T>(sys, x, q, boxes, grid, sy, u - sys[sy].gather_off, sh, st[threadIdx.x >> 5]);
-  }
-}
-
-// partials: kBatchPmeMaxBlocks per system; tickets and energies: 2 per system
-// ([2s] reciprocal, [2s+1] self).
-template <class T>
-__global__ void __launch_bounds__(kPmeBlock, 4) batch_convolve_kernel(const BatchSys *sys, const BatchShape *shape,
-                                                                   typename CplxOf<T>::type *S, const T *boxes,
-                                                                   double alpha, const T *moduli, double *partials,
-                                                                   unsigned *tickets, double *energies,
-                                                                   unsigned *counter) {
-  __shared__ PmeShared sh;
-  const int nsys = shape->nsys, units = shape->conv_units;
-  for (int u = next_unit(counter); u < units; u = next_unit(counter)) {
-    const int sy = unit_system<kUnitsConv>(sys, nsys, u);
-    const BatchSys &b = sys[sy];
-    const int bx = u - b.conv_off;
-    if (threadIdx.x == 0) load_pme_shared(boxes + 9 * (int64_t)sy, b.K, sh);
-    __syncthreads();
-    const T *xm = moduli + b.mod_off, *ym = xm + b.K, *zm = ym + b.K;
-    const double e = convolve_points<T>(S + b.cplx_off, sh, b.K, alpha, xm, ym, zm, bx, b.conv_blocks);
-    grid_sum_n<kPmeBlock>(0.5 * e, partials + (int64_t)kBatchPmeMaxBlocks * sy, tickets + 2 * sy, energies + 2 * sy,
-                          false, bx, b.conv_blocks);
   }
 }
 
@@ -961,7 +739,9 @@ struct PmePlanImpl {
   int dtype;
   int K;
   int device;
-  cufftHandle r2c, c2r;
+  bool planes;              // solved by the plane kernels (pme_fft.cuh), else by cuFFT
+  void *tables = nullptr;   // planes: the tables of side K (fft_table)
+  cufftHandle r2c, c2r;     // cuFFT plans otherwise
 };
 
 int pme_cufft_fail(cufftResult r, const char *what);
@@ -976,49 +756,10 @@ namespace tff {
 
 // FFT -> convolve -> FFT of the spread grid in ws (L.fix) on `s`; leaves the potential grid
 // Phi in (T*)(ws + L.real) (mixed) or (T*)(ws + L.fix) (FP64), returned through *phi_grid.
+// after_kernel: the work before it on the stream is a kernel. Defined in pme.cu.
 template <class T>
 int pme_solve_phase(const PmePlanImpl &p, const PmeLayout &L, char *ws, const T *box, double alpha, const T *xmod,
-                    const T *ymod, const T *zmod, cudaStream_t s, T **phi_grid) {
-  using S = typename Acc<T>::S;
-  const int K = p.K;
-  const int sms = sm_count();
-  S *grid = reinterpret_cast<S *>(ws + L.fix);
-  T *real;
-  if (sizeof(T) == 4) {
-    real = reinterpret_cast<T *>(ws + L.real);
-    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((L.ngrid + 255) / 256, sms * 8));
-    pme_fix_to_real_kernel<<<nb, 256, 0, s>>>(reinterpret_cast<unsigned long long *>(grid),
-                                              reinterpret_cast<float *>(real), L.ngrid);
-    TFF_LAUNCHED();
-  } else {
-    real = reinterpret_cast<T *>(grid);
-  }
-  auto *cplx = reinterpret_cast<typename CplxOf<T>::type *>(ws + L.cplx);
-  cufftResult r;
-  if ((r = cufftSetStream(p.r2c, s)) != CUFFT_SUCCESS) return pme_cufft_fail(r, "cufftSetStream");
-  if ((r = cufftSetStream(p.c2r, s)) != CUFFT_SUCCESS) return pme_cufft_fail(r, "cufftSetStream");
-  if (sizeof(T) == 4)
-    r = cufftExecR2C(p.r2c, reinterpret_cast<cufftReal *>(real), reinterpret_cast<cufftComplex *>(cplx));
-  else
-    r = cufftExecD2Z(p.r2c, reinterpret_cast<cufftDoubleReal *>(real), reinterpret_cast<cufftDoubleComplex *>(cplx));
-  if (r != CUFFT_SUCCESS) return pme_cufft_fail(r, "forward FFT");
-  double *partials = reinterpret_cast<double *>(ws + L.partials);
-  unsigned *tickets = reinterpret_cast<unsigned *>(ws + L.tickets);
-  double *energies = reinterpret_cast<double *>(ws + L.energies);
-  {
-    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((L.ncplx + kPmeBlock - 1) / kPmeBlock, sms * 4));
-    pme_convolve_kernel<T><<<nb, kPmeBlock, 0, s>>>(cplx, box, K, alpha, xmod, ymod, zmod, partials, tickets,
-                                                    energies);
-    TFF_LAUNCHED();
-  }
-  if (sizeof(T) == 4)
-    r = cufftExecC2R(p.c2r, reinterpret_cast<cufftComplex *>(cplx), reinterpret_cast<cufftReal *>(real));
-  else
-    r = cufftExecZ2D(p.c2r, reinterpret_cast<cufftDoubleComplex *>(cplx), reinterpret_cast<cufftDoubleReal *>(real));
-  if (r != CUFFT_SUCCESS) return pme_cufft_fail(r, "inverse FFT");
-  *phi_grid = real;
-  return TFF_OK;
-}
+                    const T *ymod, const T *zmod, cudaStream_t s, T **phi_grid, bool after_kernel = true);
 
 // Enqueue spread -> FFT -> convolve -> FFT on `s` (see pme_solve_phase for the result).
 template <class T, class Atoms>
@@ -1031,7 +772,7 @@ int pme_grid_phase(const PmePlanImpl &p, const PmeLayout &L, char *ws, Atoms ato
     pme_spread_kernel<T, Atoms><<<pme_blocks(nthreads), kPmeBlock, 0, s>>>(atoms, nthreads, box, p.K, grid);
     TFF_LAUNCHED();
   }
-  return pme_solve_phase<T>(p, L, ws, box, alpha, xmod, ymod, zmod, s, phi_grid);
+  return pme_solve_phase<T>(p, L, ws, box, alpha, xmod, ymod, zmod, s, phi_grid, nthreads > 0);
 }
 
 template <class T, class Atoms, class Out>

@@ -402,7 +402,7 @@ int tff_server_create(const tff_server_desc *desc, tff_server *out) {
     if (st == TFF_OK && e == cudaSuccess) e = cudaMallocHost((void **)&l.h_out, l.out_bytes);
     if (st == TFF_OK && e == cudaSuccess) e = cudaMalloc((void **)&l.d_in, l.in_bytes);
     if (st == TFF_OK && e == cudaSuccess) e = cudaMalloc((void **)&l.d_out, l.out_bytes);
-    // the lane's staging buffers never change: its graph of the common DFT class is
+    // the lane's staging buffers never change: its graph of the common transform class is
     // captured now rather than on the way of the first requests
     if (st == TFF_OK && e == cudaSuccess)
       st = batch_warm_graph(l.batch, l.d_in + l.o_x, l.d_in + l.o_box, l.d_in + l.o_q, l.d_in + l.o_s,
