@@ -51,9 +51,8 @@ inline int table_offset(int K) {
 
 // Bytes before the system table in the uploaded block (the BatchShape sits there).
 constexpr size_t kTableOffset = 256;
-// Atoms (sorted slots) of a batched gather work unit: four passes of a 256-thread block at
-// 5 atoms per warp.
-constexpr int64_t kGatherAtomsPerUnit = 4 * (256 / 32) * 5;
+// Atoms (sorted slots) of a batched gather work unit: five passes of a 256-thread block.
+constexpr int64_t kGatherAtomsPerUnit = 5 * (256 / 32) * kGatherAtoms;
 static_assert(sizeof(BatchShape) <= kTableOffset, "BatchShape must fit before the system table");
 
 struct BatchLayout {
