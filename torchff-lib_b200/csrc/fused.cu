@@ -158,7 +158,8 @@ int system_eval_impl(tff_system sys, const T *x, const T *box, double *energy, T
     const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((sys->cl.npad + 255) / 256, sms * 8));
     st = launch_k(pdl, sorted_params_kernel<T>, nb, 256, 0, s, cd, static_cast<const T *>(sys->sigma),
                   static_cast<const T *>(sys->eps), static_cast<const int *>(sys->excl), lj, sys->exslot,
-                  static_cast<const T *>(nullptr), static_cast<typename V4<T>::type *>(nullptr), gx, gq);
+                  static_cast<const T *>(nullptr), static_cast<typename V4<T>::type *>(nullptr), gx, gq,
+                  static_cast<S *>(nullptr));
     if (st != TFF_OK) return st;
     TileArgs<T> A;
     A.cl = cd;
@@ -198,6 +199,7 @@ __global__ void finalize_grads_kernel(ClusterData<T> cl, const typename Acc<T>::
                                       const T *pme_scal, const T *eps, double kc, T *out_x, T *out_q, T *out_s,
                                       T *out_e, const typename Acc<T>::S *e_tile, const double *e_pme,
                                       double *energy, const typename Acc<T>::S *bonded) {
+  pdl_enter();
   using S = typename Acc<T>::S;
   const int64_t np = cl.npad;
   const S *gx = acc, *gq = acc + 3 * np, *gs = acc + 4 * np, *ga = acc + 5 * np;
@@ -240,7 +242,6 @@ int system_grad_impl(tff_system sys, const T *x, const T *box, const T *dir, dou
   }
   const int sms = sm_count();
   S *energies = reinterpret_cast<S *>(sys->scratch);
-  TFF_CUDA(cudaMemsetAsync(sys->scratch, 0, 8 * sizeof(double), s));
   const bool use_pme = sys->pme && n > 0;
   const double *e_pme = nullptr;
   if (MODE == 1 && !use_pme && sys->has_bonded() && n > 0) {
@@ -263,7 +264,6 @@ int system_grad_impl(tff_system sys, const T *x, const T *box, const T *dir, dou
     int st = pme_grid_phase<T>(sys->pme->impl, sys->pl, pw, atoms, n, box, sys->desc.ewald_alpha, xm, ym, zm, ps,
                                &phi_grid);
     if (st != TFF_OK) return st;
-    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((n * kLanesPerAtom + kPmeBlock - 1) / kPmeBlock, sms * 8));
     if constexpr (MODE == 1) {
       PlainGatherOut<T> out{static_cast<T *>(sys->pme_phi), static_cast<T *>(sys->pme_grad)};
       st = pme_gather_phase<T>(sys->pme->impl, sys->pl, pw, atoms, n, box, sys->desc.ewald_alpha, phi_grid, out, 1.0,
@@ -279,6 +279,7 @@ int system_grad_impl(tff_system sys, const T *x, const T *box, const T *dir, dou
       T *psi_grid = nullptr;
       st = pme_solve_phase<T>(sys->pme->impl, sys->pl, pw2, box, sys->desc.ewald_alpha, xm, ym, zm, ps, &psi_grid);
       if (st != TFF_OK) return st;
+      const int nb = pme_blocks((n + kAtomsPerWarp - 1) / kAtomsPerWarp);
       pme_gather_hvp_kernel<T><<<nb, kPmeBlock, 0, ps>>>(atoms, dir, n, box, K, phi_grid, psi_grid,
                                                          sys->desc.coul_constant, static_cast<T *>(sys->pme_hx),
                                                          static_cast<T *>(sys->pme_hq));
@@ -287,18 +288,21 @@ int system_grad_impl(tff_system sys, const T *x, const T *box, const T *dir, dou
     TFF_CUDA(cudaEventRecord(sys->join_ev, ps));
   }
   ClusterData<T> cd = cluster_data<T>(sys->cl, sys->cl_ws);
-  int st = build_clusters<T>(sys->cl, cd, sys->cl_ws, x, static_cast<const T *>(sys->q), box, sys->desc.cutoff, 0, s);
+  // one run of programmatic dependent launches, as in the energy evaluation; the build zeroes the
+  // energy accumulators, the sorted parameters the per-slot ones
+  int st = build_clusters<T>(sys->cl, cd, sys->cl_ws, x, static_cast<const T *>(sys->q), box, sys->desc.cutoff, 0, s,
+                             sys->scratch, 8 * sizeof(double), true);
   if (st != TFF_OK) return st;
   S *acc = static_cast<S *>(sys->acc);
   const int64_t np = sys->cl.npad;
-  TFF_CUDA(cudaMemsetAsync(sys->acc, 0, (size_t)np * 6 * 8, s));
   auto *lj = static_cast<typename V2<T>::type *>(sys->lj);
   auto *dsorted = static_cast<typename V4<T>::type *>(sys->dir_sorted);
   if (n > 0) {
     const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((np + 255) / 256, sms * 8));
-    sorted_params_kernel<T><<<nb, 256, 0, s>>>(cd, static_cast<const T *>(sys->sigma), static_cast<const T *>(sys->eps),
-                                               sys->excl, lj, sys->exslot, MODE == 2 ? dir : nullptr, dsorted);
-    TFF_LAUNCHED();
+    st = launch_k(true, sorted_params_kernel<T>, nb, 256, 0, s, cd, static_cast<const T *>(sys->sigma),
+                  static_cast<const T *>(sys->eps), static_cast<const int *>(sys->excl), lj, sys->exslot,
+                  MODE == 2 ? dir : static_cast<const T *>(nullptr), dsorted, acc, acc + 3 * np, acc + 4 * np);
+    if (st != TFF_OK) return st;
     TileArgs<T> A;
     A.cl = cd;
     A.lj = lj;
@@ -313,23 +317,17 @@ int system_grad_impl(tff_system sys, const T *x, const T *box, const T *dir, dou
     A.kc = sys->desc.coul_constant;
     A.energies = energies;
     const int64_t max_items = item_capacity(sys->cl.nclusters, sys->cl.cap);
-    constexpr int NW = TileCfg<T, MODE>::NW;
-    const int nbt = (int)std::max<int64_t>(1, std::min<int64_t>((max_items + NW - 1) / NW, (int64_t)sms * 48 / NW));
-    tile_kernel<T, MODE><<<nbt, NW * kWarp, 0, s>>>(A);
-    TFF_LAUNCHED();
+    if ((st = launch_tile<T, MODE>(true, max_items, sms, s, A)) != TFF_OK) return st;
   }
   if (use_pme) TFF_CUDA(cudaStreamWaitEvent(s, sys->join_ev, 0));
   const T *pvec = use_pme ? static_cast<const T *>(MODE == 1 ? sys->pme_grad : sys->pme_hx) : nullptr;
   const T *pscal = use_pme ? static_cast<const T *>(MODE == 1 ? sys->pme_phi : sys->pme_hq) : nullptr;
   const int nbf = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, sms * 8));
-  finalize_grads_kernel<T, MODE><<<nbf, 256, 0, s>>>(cd, acc, pvec, pscal, static_cast<const T *>(sys->eps),
-                                                     sys->desc.coul_constant, out_x, out_q, out_s, out_e, energies,
-                                                     e_pme, energy,
-                                                     MODE == 1 && sys->has_bonded() && n > 0
-                                                         ? static_cast<const S *>(sys->bacc)
-                                                         : nullptr);
-  TFF_LAUNCHED();
-  return TFF_OK;
+  return launch_k(true, finalize_grads_kernel<T, MODE>, nbf, 256, 0, s, cd, static_cast<const S *>(acc), pvec, pscal,
+                  static_cast<const T *>(sys->eps), sys->desc.coul_constant, out_x, out_q, out_s, out_e,
+                  static_cast<const S *>(energies), e_pme, energy,
+                  MODE == 1 && sys->has_bonded() && n > 0 ? static_cast<const S *>(sys->bacc)
+                                                          : static_cast<const S *>(nullptr));
 }
 
 template <class T>

@@ -564,9 +564,7 @@ int launch_real_space(bool pdl, int64_t max_items, int sms, cudaStream_t s, cons
     return launch_k(pdl, pair_tile_kernel<T, NW, PairTileOcc<T>::min_blocks>, nbt, NW * kWarp, 0, s, A,
                     pair_const<T>(A.alpha));
   } else {
-    constexpr int NW = TileCfg<T>::NW;
-    const int nbt = (int)std::max<int64_t>(1, std::min<int64_t>((max_items + NW - 1) / NW, (int64_t)sms * 48 / NW));
-    return launch_k(pdl, tile_kernel<T, 0>, nbt, NW * kWarp, 0, s, A);
+    return launch_tile<T, 0>(pdl, max_items, sms, s, A);
   }
 }
 

@@ -19,6 +19,7 @@
 #include <algorithm>
 
 #include "cluster.cuh"
+#include "erf_poly.cuh"
 
 namespace tff {
 namespace {
@@ -158,7 +159,8 @@ constexpr int kStagedRows = kWarp * kMaxPairIters + kWarp * kMaxPairIters / 8;
 // One atomic per value, eight memory clears and conversions per call before: a call over 20.8 M
 // rows (99,000 atoms, FP32) 1,015 -> 515 us, 1.9 M rows of LJ and Ewald (9,000 atoms) 115 and
 // 122 -> 42 and 60 us.
-template <class T, int CM, int LM>
+// ERF (FP64 Ewald): how erfc is evaluated (erf_poly.cuh).
+template <class T, int CM, int LM, int ERF>
 __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
   pdl_enter();
   using A = Acc<T>;
@@ -189,6 +191,7 @@ __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
   const T inv_rc = T(1) / rc;
   const T alpha = (T)a.alpha;
   const T two_a_rpi = (T)(2.0 * a.alpha / 1.7724538509055160273);
+  const EwaldPoly<ERF == kErfLibrary ? kErfShort : ERF> ewald(a.alpha);  // unused with kErfLibrary
   double e_acc = 0.0;
   const bool grads = a.acc != nullptr, lj_grads = kLj && a.acc_lj != nullptr;
 
@@ -257,7 +260,11 @@ __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
         const T r2 = dx * dx + dy * dy + dz * dz;
         in = r2 <= rc2;
         if (in) {
-          const T rinv = rsqrt_t(r2);
+          T rinv;
+          if constexpr (ERF != kErfLibrary)
+            rinv = rsqrt_t(r2);
+          else
+            rinv = rsqrt_t(r2);
           const T rinv2 = rinv * rinv;
           T e = T(0);
           T dedr_over_r = T(0);  // (dE/dr) / r
@@ -272,6 +279,13 @@ __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
             } else if (CM == C_PLAIN) {
               f = rinv;
               dfdr_r = -rinv2 * rinv;
+            } else if constexpr (ERF != kErfLibrary) {
+              T g;
+              if (is_excl)
+                ewald.excluded(r2, f, g);
+              else
+                ewald.eval(r2, rinv, rinv2, f, g);
+              dfdr_r = -g;
             } else {
               const T r = r2 * rinv;
               const T u = alpha * r;
@@ -465,12 +479,12 @@ int grid_blocks(int64_t work) {
   return (int)std::min(want, cap);
 }
 
-template <class T, int CM, int LM>
+template <class T, int CM, int LM, int ERF = kErfLibrary>
 int launch_pairs(PairArgs<T> a, int64_t total, cudaStream_t s) {
   const int nb = grid_blocks(total);
   const int64_t share = (total + (int64_t)nb * kPairBlock - 1) / ((int64_t)nb * kPairBlock);
   a.iters = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxPairIters, share));
-  return launch_k(true, pair_kernel<T, CM, LM>, nb, kPairBlock, 0, s, a);
+  return launch_k(true, pair_kernel<T, CM, LM, ERF>, nb, kPairBlock, 0, s, a);
 }
 
 template <class T>
@@ -481,6 +495,12 @@ int dispatch_pairs(int cm, int lm, const PairArgs<T> &a, int64_t total, cudaStre
   TFF_PAIR_CASE(C_PLAIN, L_ATOM)
   TFF_PAIR_CASE(C_SHIFT, L_NONE)
   TFF_PAIR_CASE(C_PLAIN, L_NONE)
+  if constexpr (sizeof(T) == 8)
+    if (cm == C_EWALD && lm == L_NONE) {
+      const ErfRange range = erf_range(a.alpha, a.rc);
+      if (range == kErfShort) return launch_pairs<T, C_EWALD, L_NONE, kErfShort>(a, total, s);
+      if (range == kErfLong) return launch_pairs<T, C_EWALD, L_NONE, kErfLong>(a, total, s);
+    }
   TFF_PAIR_CASE(C_EWALD, L_NONE)
   TFF_PAIR_CASE(C_NONE, L_PAIR)
   TFF_PAIR_CASE(C_NONE, L_TYPE)

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "bonded.cuh"
+#include "erf_poly.cuh"
 #include "pme.cuh"
 
 namespace tff {
@@ -74,14 +75,15 @@ struct TileArgs {
 // from the first atom of the atom's own system (batch mode), i.e. global for one system.
 // With `dir` (caller order (N,3)) also the direction of a second-derivative pass in
 // sorted order.
-// With `gx` / `gq` also zeroes the tile kernel's accumulators of each slot (3 + 1 values).
+// With `gx` / `gq` also zeroes the tile kernel's accumulators of each slot (3 + 1 values, with
+// `gp` the npad slots of each parameter derivative too).
 // Also fills the tile kernel's item -> cluster table from the item offsets of the
 // neighbour search (the lanes of cluster k write its entries).
 template <class T>
 __global__ void sorted_params_kernel(ClusterData<T> cl, const T *sigma, const T *eps, const int *excl,
                                      typename V2<T>::type *lj, int *exslot, const T *dir = nullptr,
                                      typename V4<T>::type *dir_sorted = nullptr, typename Acc<T>::S *gx = nullptr,
-                                     typename Acc<T>::S *gq = nullptr) {
+                                     typename Acc<T>::S *gq = nullptr, typename Acc<T>::S *gp = nullptr) {
   pdl_enter();
   const int64_t npad = cl.n_pad();
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < npad; s += (int64_t)gridDim.x * blockDim.x) {
@@ -91,6 +93,7 @@ __global__ void sorted_params_kernel(ClusterData<T> cl, const T *sigma, const T 
       gx[3 * s + 2] = 0;
       gq[s] = 0;
     }
+    if (gp) gp[s] = gp[npad + s] = 0;
     {
       const int64_t k = s / kWarp;
       const int o = cl.itemoff[k], nk = cl.itemoff[k + 1] - o;
@@ -121,12 +124,13 @@ __device__ __forceinline__ void pair_min_image(bool ortho, T &dx, T &dy, T &dz, 
   }
 }
 
-// Resident 4-warp blocks per SM the register allocation of the energy kernel must allow
-// (6 blocks = 24 warps: at most 80 registers per thread).
-constexpr int kTileMinBlocks = 6;
+// Resident 2-warp blocks per SM the register allocation of the FP64 energy kernel must allow: 10 (at
+// most 96 registers). 3000 waters: 141 us per evaluation, 147 at 6 (104 registers), 150 at 13 (72).
+constexpr int kTileMinBlocks = 10;
 
-template <class T, int MODE = 0, int MIN_BLOCKS = kTileMinBlocks>
-__global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? MIN_BLOCKS : 1)
+// ERF (FP64): how the screened Coulomb terms are evaluated (erf_poly.cuh).
+template <class T, int MODE = 0, int ERF = kErfLibrary>
+__global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? kTileMinBlocks : 1)
     tile_kernel(TileArgs<T> A) {
   pdl_enter();
   using V = typename V4<T>::type;
@@ -154,6 +158,7 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? MIN_BLO
   const T alpha = (T)A.alpha;
   const T kc = (T)A.kc;
   const T two_a_rpi = (T)(2.0 * A.alpha / 1.7724538509055160273);
+  const EwaldPoly<ERF == kErfLibrary ? kErfShort : ERF> ewald(A.alpha);  // unused with kErfLibrary
 
   const int nitems = cl.itemoff[cl.n_clusters()];
   const int nwarps = gridDim.x * NW;
@@ -337,94 +342,7 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? MIN_BLO
     T fx = T(0), fy = T(0), fz = T(0), dq = T(0);
     double ep = 0.0;
     T d_sig = T(0), d_a = T(0);  // MODE 1/2: sigma and sqrt(eps) derivatives of atom i
-    if constexpr (MODE == 0 && sizeof(T) == 4) {
-      // FP32: two pairs per iteration with paired instructions (FADD2/FMUL2/FFMA2); only
-      // rsqrt, reciprocal and exp2 stay scalar. A lane with an odd count pads the second
-      // slot with a zero-charge, zero-epsilon copy of the first, which contributes nothing.
-      const float2 one2 = make_float2(1.f, 1.f), mone2 = make_float2(-1.f, -1.f);
-      const float2 al2 = make_float2(alpha, alpha), ta2 = make_float2(two_a_rpi, two_a_rpi);
-      const float2 nkq2 = make_float2(-kqi, -kqi), kq2 = make_float2(kqi, kqi);
-      const float2 pix = make_float2(pi.x, pi.x), piy = make_float2(pi.y, pi.y), piz = make_float2(pi.z, pi.z);
-      const float2 sgi = make_float2(lji.x, lji.x), epi = make_float2(lji.y, lji.y);
-      float2 fx2 = make_float2(0.f, 0.f), fy2 = fx2, fz2 = fx2, dq2 = fx2, te2 = fx2;
-      int t = 0, iter = 0;
-      unsigned m = ntile > 0 ? s_mask[w][0][lane] : 0u;
-      while (true) {
-        int ta = 0, sa = 0, tb = 0, sb = 0;
-        while (m == 0u && ++t < ntile) m = s_mask[w][t][lane];
-        const bool ha = m != 0u;
-        if (ha) {
-          sa = __ffs(m) - 1;
-          m &= m - 1u;
-          ta = t;
-        }
-        while (m == 0u && ++t < ntile) m = s_mask[w][t][lane];
-        const bool hb = m != 0u;
-        if (hb) {
-          sb = __ffs(m) - 1;
-          m &= m - 1u;
-          tb = t;
-        }
-        if (!__any_sync(kFull, ha)) break;
-        if ((++iter & 15) == 0) {
-          ep += (double)(te2.x + te2.y);
-          te2 = make_float2(0.f, 0.f);
-        }
-        if (ha) {
-          const float4 qa = s_pos[w][ta][sa];
-          float4 qb = hb ? s_pos[w][tb][sb] : make_float4(qa.x, qa.y, qa.z, 0.f);
-          const float2 la = s_lj[w][ta][sa];
-          const float2 lb = hb ? s_lj[w][tb][sb] : make_float2(0.f, 0.f);
-          float2 dx = __fadd2_rn(pix, make_float2(-qa.x, -qb.x));
-          float2 dy = __fadd2_rn(piy, make_float2(-qa.y, -qb.y));
-          float2 dz = __fadd2_rn(piz, make_float2(-qa.z, -qb.z));
-          if (!all_shifted) {
-            if (s_mi[w][ta]) pair_min_image(ortho, dx.x, dy.x, dz.x, s_m, s_inv);
-            if (hb && s_mi[w][tb]) pair_min_image(ortho, dx.y, dy.y, dz.y, s_m, s_inv);
-          }
-          float2 r2 = __fmul2_rn(dx, dx);
-          r2 = __ffma2_rn(dy, dy, r2);
-          r2 = __ffma2_rn(dz, dz, r2);
-          const float2 rinv = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-          const float2 rinv2 = __fmul2_rn(rinv, rinv);
-          const float2 u = __fmul2_rn(__fmul2_rn(r2, rinv), al2);
-          // erfc(u) exp(u^2) by Abramowitz & Stegun 7.1.26 (see erfc_exp_as)
-          const float2 den = __ffma2_rn(u, make_float2(0.3275911f, 0.3275911f), one2);
-          const float2 tt = make_float2(__fdividef(1.f, den.x), __fdividef(1.f, den.y));
-          float2 poly = __ffma2_rn(tt, make_float2(1.061405429f, 1.061405429f),
-                                   make_float2(-1.453152027f, -1.453152027f));
-          poly = __ffma2_rn(tt, poly, make_float2(1.421413741f, 1.421413741f));
-          poly = __ffma2_rn(tt, poly, make_float2(-0.284496736f, -0.284496736f));
-          poly = __ffma2_rn(tt, poly, make_float2(0.254829592f, 0.254829592f));
-          poly = __fmul2_rn(tt, poly);
-          const float2 mu2 = __fmul2_rn(u, u);
-          const float2 ex = make_float2(__expf(-mu2.x), __expf(-mu2.y));
-          const float2 ec = __fmul2_rn(poly, ex);
-          const float2 qj = make_float2(qa.w, qb.w);
-          const float2 cq = __fmul2_rn(__fmul2_rn(qj, ec), rinv);  // E_coul / (k q_i)
-          const float2 g = __ffma2_rn(ta2, __fmul2_rn(ex, rinv), __fmul2_rn(ec, rinv2));
-          float2 dedr = __fmul2_rn(__fmul2_rn(g, rinv), __fmul2_rn(qj, nkq2));
-          const float2 sig = __fadd2_rn(sgi, make_float2(la.x, lb.x));
-          const float2 eps = __fmul2_rn(epi, make_float2(la.y, lb.y));
-          const float2 sr2 = __fmul2_rn(__fmul2_rn(sig, sig), rinv2);
-          const float2 sr6 = __fmul2_rn(__fmul2_rn(sr2, sr2), sr2);
-          const float2 es6 = __fmul2_rn(eps, sr6);
-          dedr = __ffma2_rn(__fmul2_rn(es6, make_float2(-24.f, -24.f)),
-                            __fmul2_rn(__ffma2_rn(sr6, make_float2(2.f, 2.f), mone2), rinv2), dedr);
-          fx2 = __ffma2_rn(dedr, dx, fx2);
-          fy2 = __ffma2_rn(dedr, dy, fy2);
-          fz2 = __ffma2_rn(dedr, dz, fz2);
-          dq2 = __fadd2_rn(dq2, cq);
-          te2 = __ffma2_rn(cq, kq2, te2);
-          te2 = __ffma2_rn(__fmul2_rn(es6, make_float2(4.f, 4.f)), __fadd2_rn(sr6, mone2), te2);
-        }
-      }
-      ep += (double)(te2.x + te2.y);
-      fx = fx2.x + fx2.y;
-      fy = fy2.x + fy2.y;
-      fz = fz2.x + fz2.y;
-      dq = dq2.x + dq2.y;
-    } else if constexpr (MODE != 0) {
+    if constexpr (MODE != 0) {
       // one pair per step. With D = (dE/dr)/r of the pair: MODE 1 adds dE/dsigma_i and
       // dE/da_i; MODE 2 accumulates, with delta = u_i - u_j and rd = r_ij . delta,
       // d/dx_i (u . dE/dx) = D delta + (dD/dr / r) rd r_ij and the parameter derivatives
@@ -448,22 +366,37 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? MIN_BLO
           T dx = pi.x - q.x, dy = pi.y - q.y, dz = pi.z - q.z;
           if (s_mi[w][t]) pair_min_image(ortho, dx, dy, dz, s_m, s_inv);
           const T r2 = dx * dx + dy * dy + dz * dz;
-          const T rinv = rsqrt_t(r2);
-          const T rinv2 = rinv * rinv;
-          const T u = alpha * (r2 * rinv);
-          T ec, ex2;
-          erfc_exp(u, ec, ex2);
+          // f = erfc(alpha r) / r, g = -(1/r) df/dr, h = -(1/r) dg/dr (MODE 2)
+          T rinv, rinv2, f, g, h = T(0);
+          if constexpr (ERF != kErfLibrary) {
+            rinv = rsqrt_t(r2);
+            rinv2 = rcp_newton(r2, rinv);
+            ewald.eval(r2, rinv, rinv2, f, g);
+            if constexpr (MODE == 2) h = ewald.second(r2, rinv, rinv2);
+          } else {
+            rinv = rsqrt_t(r2);
+            rinv2 = rinv * rinv;
+            const T u = alpha * (r2 * rinv);
+            T ec, ex2;
+            erfc_exp(u, ec, ex2);
+            f = ec * rinv;
+            g = (ec * rinv2 + two_a_rpi * ex2 * rinv) * rinv;
+            if constexpr (MODE == 2) {
+              const T rinv4 = rinv2 * rinv2;
+              h = T(3) * ec * rinv4 * rinv + two_a_rpi * ex2 * (T(3) * rinv4 + T(2) * alpha * alpha * rinv2);
+            }
+          }
           const T sig = lji.x + ljj.x, aj = ljj.y, eps = lji.y * aj;
           const T sr = sig * rinv, sr2 = sr * sr, sr6 = sr2 * sr2 * sr2, sr12 = sr6 * sr6, s5 = sr2 * sr2 * sr;
-          const T dcq = -q.w * (ec * rinv2 + two_a_rpi * ex2 * rinv) * rinv;  // D_coulomb / (k q_i)
+          const T dcq = -q.w * g;  // D_coulomb / (k q_i)
           const T dlj = T(-24) * eps * (T(2) * sr12 - sr6) * rinv2;           // D_lj
           const T D = kqi * dcq + dlj;
           if constexpr (MODE == 1) {
             fx += D * dx;
             fy += D * dy;
             fz += D * dz;
-            dq += q.w * ec * rinv;
-            te += kqi * q.w * ec * rinv + T(4) * eps * (sr12 - sr6);
+            dq += q.w * f;
+            te += kqi * q.w * f + T(4) * eps * (sr12 - sr6);
             d_sig += T(12) * eps * rinv * s5 * (T(2) * sr6 - T(1));  // 1/2 dE/dsigma_ij
             d_a += T(4) * aj * (sr12 - sr6);                       // dE/da_i
           } else {
@@ -471,7 +404,7 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? MIN_BLO
             const T ddx = ui.x - uj.x, ddy = ui.y - uj.y, ddz = ui.z - uj.z;
             const T rd = dx * ddx + dy * ddy + dz * ddz;
             const T rinv4 = rinv2 * rinv2;
-            const T e2 = kqi * q.w * (T(3) * ec * rinv4 * rinv + two_a_rpi * ex2 * (T(3) * rinv4 + T(2) * alpha * alpha * rinv2)) +
+            const T e2 = kqi * q.w * h +
                          T(24) * eps * (T(28) * sr12 - T(8) * sr6) * rinv4;  // (dD/dr) / r
             const T e2rd = e2 * rd;
             fx += D * ddx + e2rd * dx;
@@ -504,13 +437,22 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? MIN_BLO
           T dx = pi.x - q.x, dy = pi.y - q.y, dz = pi.z - q.z;
           if (s_mi[w][t]) pair_min_image(ortho, dx, dy, dz, s_m, s_inv);
           const T r2 = dx * dx + dy * dy + dz * dz;
-          const T rinv = rsqrt_t(r2);
-          const T rinv2 = rinv * rinv;
-          const T u = alpha * (r2 * rinv);
-          T ec, ex2;
-          erfc_exp(u, ec, ex2);
-          const T cq = q.w * ec * rinv;  // E_coul / (k q_i)
-          T dedr_r = -kqi * q.w * (ec * rinv2 + two_a_rpi * ex2 * rinv) * rinv;
+          T rinv, rinv2, f, g;
+          if constexpr (ERF != kErfLibrary) {
+            rinv = rsqrt_t(r2);
+            rinv2 = rcp_newton(r2, rinv);
+            ewald.eval(r2, rinv, rinv2, f, g);
+          } else {
+            rinv = rsqrt_t(r2);
+            rinv2 = rinv * rinv;
+            const T u = alpha * (r2 * rinv);
+            T ec, ex2;
+            erfc_exp(u, ec, ex2);
+            f = ec * rinv;
+            g = (ec * rinv2 + two_a_rpi * ex2 * rinv) * rinv;
+          }
+          const T cq = q.w * f;  // E_coul / (k q_i)
+          T dedr_r = -kqi * q.w * g;
           const T sig = lji.x + ljj.x;
           const T eps = lji.y * ljj.y;
           const T sr2 = sig * sig * rinv2;
@@ -541,20 +483,32 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? MIN_BLO
         T dx = pi.x - q.x, dy = pi.y - q.y, dz = pi.z - q.z;
         if (s_mi[w][t]) pair_min_image(ortho, dx, dy, dz, s_m, s_inv);
         const T r2 = dx * dx + dy * dy + dz * dz;
-        const T rinv = rsqrt_t(r2);
-        const T u = alpha * (r2 * rinv);
-        const T damp = -erf_t(u);
-        const T ex2 = exp(-u * u);
-        const T cq = q.w * damp * rinv;
-        const T dcq = -q.w * (damp * rinv * rinv + two_a_rpi * ex2 * rinv) * rinv;
+        // f = -erf(alpha r) / r, g = -(1/r) df/dr, h = -(1/r) dg/dr (MODE 2)
+        T f, g, h = T(0);
+        if constexpr (ERF != kErfLibrary) {
+          ewald.excluded(r2, f, g);
+          if constexpr (MODE == 2) h = ewald.excluded_second(r2);
+        } else {
+          const T rinv = rsqrt_t(r2);
+          const T u = alpha * (r2 * rinv);
+          const T damp = -erf_t(u);
+          const T ex2 = exp(-u * u);
+          f = damp * rinv;
+          g = (damp * rinv * rinv + two_a_rpi * ex2 * rinv) * rinv;
+          if constexpr (MODE == 2) {
+            const T rinv2 = rinv * rinv, rinv4 = rinv2 * rinv2;
+            h = T(3) * damp * rinv4 * rinv + two_a_rpi * ex2 * (T(3) * rinv4 + T(2) * alpha * alpha * rinv2);
+          }
+        }
+        const T cq = q.w * f;
+        const T dcq = -q.w * g;
         const T dedr_r = kqi * dcq;
         if constexpr (MODE == 2) {
           // same form as the erfc term with erfc(u) -> erfc(u) - 1 (equal derivatives)
           const V uj = s_u[w][t][s];
           const T ddx = ui.x - uj.x, ddy = ui.y - uj.y, ddz = ui.z - uj.z;
           const T rd = dx * ddx + dy * ddy + dz * ddz;
-          const T rinv2 = rinv * rinv, rinv4 = rinv2 * rinv2;
-          const T e2rd = kqi * q.w * (T(3) * damp * rinv4 * rinv + two_a_rpi * ex2 * (T(3) * rinv4 + T(2) * alpha * alpha * rinv2)) * rd;
+          const T e2rd = kqi * q.w * h * rd;
           fx += dedr_r * ddx + e2rd * dx;
           fy += dedr_r * ddy + e2rd * dy;
           fz += dedr_r * ddz + e2rd * dz;
@@ -666,6 +620,21 @@ __global__ void cast_inputs_kernel(const double *x64, const double *box64, T *x,
 // Host-side B-spline moduli theta(k) = sum_{m=-3}^{2} M6(m+3) cos(2 pi m k / K)
 // (torchff/bsplines.py:20-63), with M6 at the integers from the same recursion as the
 // device splines.
+// Launches the tile kernel of a mode; FP64 with the polynomial range that covers alpha rc.
+template <class T, int MODE>
+int launch_tile(bool pdl, int64_t max_items, int sms, cudaStream_t s, const TileArgs<T> &A) {
+  constexpr int NW = TileCfg<T, MODE>::NW;
+  const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((max_items + NW - 1) / NW, (int64_t)sms * 48 / NW));
+  if constexpr (sizeof(T) == 8) {
+    switch (erf_range(A.alpha, A.rc)) {
+      case kErfShort: return launch_k(pdl, tile_kernel<T, MODE, kErfShort>, nb, NW * kWarp, 0, s, A);
+      case kErfLong: return launch_k(pdl, tile_kernel<T, MODE, kErfLong>, nb, NW * kWarp, 0, s, A);
+      default: break;
+    }
+  }
+  return launch_k(pdl, tile_kernel<T, MODE, kErfLibrary>, nb, NW * kWarp, 0, s, A);
+}
+
 inline void host_bspline6_at_integers(double val[6]) {
   double m[6] = {0, 1, 0, 0, 0, 0};  // M2(0)=0, M2(1)=1
   for (int n = 3; n <= 6; ++n) {
