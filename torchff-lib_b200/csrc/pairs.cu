@@ -42,8 +42,9 @@ struct PairBox {
 
 template <class T>
 struct PairArgs {
-  const typename V4<T>::type *atoms;    // (x, y, z, charge); L_TYPE: the type index in the last word
-  const typename LjRec<T>::type *lj;    // L_ATOM: (sigma, epsilon)
+  const typename V4<T>::type *atoms;    // (x, y, z, charge); L_TYPE: the type index in the last word.
+                                        // FP32 L_ATOM: two per atom, the second (sigma, epsilon, 0, 0)
+  const typename LjRec<T>::type *lj;    // FP64 L_ATOM: (sigma, epsilon)
   const PairBox<T> *box;                // NULL: open boundaries
   const int64_t *pairs;
   int64_t npairs;
@@ -74,7 +75,8 @@ template <class T>
 __global__ void __launch_bounds__(kPairBlock) pair_prep_kernel(int64_t n, const T *x, const T *q, const int64_t *types,
                                                                const T *sig, const T *eps, const T *box,
                                                                typename V4<T>::type *atoms,
-                                                               typename LjRec<T>::type *lj, PairBox<T> *box_out,
+                                                               bool wide, typename LjRec<T>::type *lj,
+                                                               PairBox<T> *box_out,
                                                                ulonglong2 *acc, int64_t nacc2, unsigned *ticket) {
   pdl_enter();
   const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (int64_t)gridDim.x * blockDim.x;
@@ -94,7 +96,13 @@ __global__ void __launch_bounds__(kPairBlock) pair_prep_kernel(int64_t n, const 
   for (int64_t k = t0; k < nacc2; k += stride) acc[k] = make_ulonglong2(0ull, 0ull);
   for (int64_t i = t0; i < n; i += stride) {
     const T w = q ? q[i] : (types ? type_bits(T(0), (int)types[i]) : T(0));
-    atoms[i] = make_v4(x[3 * i], x[3 * i + 1], x[3 * i + 2], w);
+    const auto rec = make_v4(x[3 * i], x[3 * i + 1], x[3 * i + 2], w);
+    if (wide) {
+      atoms[2 * i] = rec;
+      atoms[2 * i + 1] = make_v4(sig[i], eps[i], T(0), T(0));
+      continue;
+    }
+    atoms[i] = rec;
     if (lj) {
       typename LjRec<T>::type r;
       r.x = sig[i];
@@ -108,11 +116,13 @@ __global__ void __launch_bounds__(kPairBlock) pair_prep_kernel(int64_t n, const 
 template <class T> struct Contrib;
 template <> struct Contrib<float> {
   using S = unsigned long long;
+  using S2 = ulonglong2;
   static __device__ __forceinline__ S of(float v) { return to_fix_f(v); }
   static __device__ __forceinline__ S minus(S v) { return 0ull - v; }
 };
 template <> struct Contrib<double> {
   using S = double;
+  using S2 = double2;
   static __device__ __forceinline__ S of(double v) { return v; }
   static __device__ __forceinline__ S minus(S v) { return -v; }
 };
@@ -127,6 +137,24 @@ __device__ __forceinline__ float rsqrt_t(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double rsqrt_t(double x) { return rsqrt(x); }
 __device__ __forceinline__ float sqrt_t(float x) { return sqrtf(x); }
 __device__ __forceinline__ double sqrt_t(double x) { return sqrt(x); }
+
+// FP32 L_ATOM calls read an atom's six operands as one 32-byte record.
+template <class T, int LM> constexpr bool kWideRec = sizeof(T) == 4 && LM == L_ATOM;
+
+// Record of atom i; `lj` only for L_ATOM.
+template <class T, int LM>
+__device__ __forceinline__ void load_atom(const PairArgs<T> &a, unsigned i, typename V4<T>::type &r,
+                                          typename LjRec<T>::type &lj) {
+  if constexpr (kWideRec<T, LM>) {
+    float u, v;
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w), "=f"(lj.x), "=f"(lj.y), "=f"(u), "=f"(v)
+                 : "l"(a.atoms + 2 * (int64_t)i));
+  } else {
+    r = a.atoms[i];
+    if (LM == L_ATOM) lj = a.lj[i];
+  }
+}
 
 // Adds the NC values of each lane's row (ids: accumulator row or kNoRow) into rows of NC
 // accumulators. 32 / NC rows go per instruction, their values on neighbouring lanes, so that the
@@ -161,7 +189,7 @@ constexpr int kStagedRows = kWarp * kMaxPairIters + kWarp * kMaxPairIters / 8;
 // 122 -> 42 and 60 us.
 // ERF (FP64 Ewald): how erfc is evaluated (erf_poly.cuh).
 template <class T, int CM, int LM, int ERF>
-__global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
+__global__ void __launch_bounds__(kPairBlock, sizeof(T) == 4 ? 4 : 3) pair_kernel(PairArgs<T> a) {
   pdl_enter();
   using A = Acc<T>;
   using C = Contrib<T>;
@@ -180,6 +208,7 @@ __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
   }
   __syncthreads();
   const bool ortho = periodic && s_box.ortho;
+  const T bx = s_box.m[0], by = s_box.m[4], bz = s_box.m[8], ix = s_box.inv[0], iy = s_box.inv[4], iz = s_box.inv[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   S *val = s_val[w];
   unsigned *ids = s_id[w];
@@ -242,29 +271,28 @@ __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
       bool in = i != kNoRow;
       T fx = T(0), fy = T(0), fz = T(0), gqi = T(0), gqj = T(0), gsv = T(0), gei = T(0), gej = T(0);
       if (in) {
-        const auto pi = a.atoms[i], pj = a.atoms[j];
+        typename V4<T>::type pi, pj;
+        typename LjRec<T>::type li{}, lj{};
+        load_atom<T, LM>(a, i, pi, li);
+        load_atom<T, LM>(a, j, pj, lj);
         T dx = pi.x - pj.x;
         T dy = pi.y - pj.y;
         T dz = pi.z - pj.z;
         if (ortho) {  // min_image without the products by zero
-          T sa = dx * s_box.inv[0], sb = dy * s_box.inv[4], sc = dz * s_box.inv[8];
+          T sa = dx * ix, sb = dy * iy, sc = dz * iz;
           sa -= floor(sa + T(0.5));
           sb -= floor(sb + T(0.5));
           sc -= floor(sc + T(0.5));
-          dx = sa * s_box.m[0];
-          dy = sb * s_box.m[4];
-          dz = sc * s_box.m[8];
+          dx = sa * bx;
+          dy = sb * by;
+          dz = sc * bz;
         } else if (periodic) {
           min_image(dx, dy, dz, s_box.m, s_box.inv);
         }
         const T r2 = dx * dx + dy * dy + dz * dz;
         in = r2 <= rc2;
         if (in) {
-          T rinv;
-          if constexpr (ERF != kErfLibrary)
-            rinv = rsqrt_t(r2);
-          else
-            rinv = rsqrt_t(r2);
+          const T rinv = rsqrt_t(r2);
           const T rinv2 = rinv * rinv;
           T e = T(0);
           T dedr_over_r = T(0);  // (dE/dr) / r
@@ -304,7 +332,6 @@ __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
             T s, ep, sqe_i = T(0), sqe_j = T(0);
             int64_t tidx = 0;
             if (LM == L_ATOM) {
-              const auto li = a.lj[i], lj = a.lj[j];
               s = T(0.5) * (li.x + lj.x);
               sqe_i = li.y;
               sqe_j = lj.y;
@@ -322,21 +349,21 @@ __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
             e += T(4) * ep * sr6 * (sr6 - T(1));
             const T g = T(24) * ep * sr6 * (T(2) * sr6 - T(1));  // = -r dE/dr = s dE/ds
             dedr_over_r -= g * rinv2;
-            const T de_ds = g / s;
-            const T de_de = T(4) * sr6 * (sr6 - T(1));
             if (LM == L_ATOM) {
-              gsv = T(0.5) * de_ds;
-              if (ep > T(0)) {
-                const T h = de_de / (T(2) * ep);
-                gei = h * sqe_j;
-                gej = h * sqe_i;
+              if (lj_grads) {
+                gsv = T(0.5) * (g / s);
+                if (ep > T(0)) {
+                  const T h = T(4) * sr6 * (sr6 - T(1)) / (T(2) * ep);
+                  gei = h * sqe_j;
+                  gej = h * sqe_i;
+                }
               }
             } else if (LM == L_PAIR) {
-              if (a.gs_pair) a.gs_pair[t] = de_ds;
-              if (a.ge_pair) a.ge_pair[t] = de_de;
+              if (a.gs_pair) a.gs_pair[t] = g / s;
+              if (a.ge_pair) a.ge_pair[t] = T(4) * sr6 * (sr6 - T(1));
             } else {
-              if (a.gs) A::add(&a.gs[tidx], (double)de_ds);
-              if (a.ge) A::add(&a.ge[tidx], (double)de_de);
+              if (a.gs) A::add(&a.gs[tidx], (double)(g / s));
+              if (a.ge) A::add(&a.ge[tidx], (double)(T(4) * sr6 * (sr6 - T(1))));
             }
           }
           e_acc += (double)e;
@@ -372,13 +399,14 @@ __global__ void __launch_bounds__(kPairBlock) pair_kernel(PairArgs<T> a) {
         ks[0] += swap ? mx : vx;
         ks[1] += swap ? my : vy;
         ks[2] += swap ? mz : vz;
-        val[4 * lane] = swap ? vx : mx;
-        val[4 * lane + 1] = swap ? vy : my;
-        val[4 * lane + 2] = swap ? vz : mz;
+        S vq = S(0);
         if (CM != C_NONE) {
           ks[3] += C::of(swap ? gqj : gqi);
-          val[4 * lane + 3] = C::of(swap ? gqi : gqj);
+          vq = C::of(swap ? gqi : gqj);
         }
+        using S2 = typename C::S2;
+        reinterpret_cast<S2 *>(val)[2 * lane] = S2{swap ? vx : mx, swap ? vy : my};
+        reinterpret_cast<S2 *>(val)[2 * lane + 1] = S2{swap ? vz : mz, vq};
         ids[lane] = other;
         __syncwarp();
         add_rows<4>(a.acc, ids, val, (lane & 3) == 3 ? CM != C_NONE && a.want_q : a.want_x, lane);
@@ -462,8 +490,8 @@ PairLayout pair_layout(int dtype, int64_t natoms, int64_t ntypes) {
   L.acc_lj = take((size_t)natoms * 2 * 8);
   L.gs_tab = take((size_t)(ntypes * ntypes) * 8);
   L.ge_tab = take((size_t)(ntypes * ntypes) * 8);
-  L.atoms = take((size_t)natoms * 4 * ts);
-  L.lj = take((size_t)natoms * 2 * ts);
+  L.atoms = take((size_t)natoms * 32);  // FP64 (x, y, z, q), or FP32 with room for a second vector
+  L.lj = take(dtype == TFF_F64 ? (size_t)natoms * 16 : 0);
   L.box = take(18 * ts + 8);
   L.partials = take(8 * 1024 * sizeof(double));
   L.ticket = take(sizeof(unsigned));
@@ -535,7 +563,8 @@ int run_pairs(const PairCall &c, cudaStream_t s) {
   char *ws = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(c.ws) + kWsAlign - 1) & ~uintptr_t(kWsAlign - 1));
   PairArgs<T> a{};
   auto *atoms = reinterpret_cast<typename V4<T>::type *>(ws + L.atoms);
-  auto *lj = c.lm == L_ATOM ? reinterpret_cast<typename LjRec<T>::type *>(ws + L.lj) : nullptr;
+  const bool wide = sizeof(T) == 4 && c.lm == L_ATOM;
+  auto *lj = c.lm == L_ATOM && !wide ? reinterpret_cast<typename LjRec<T>::type *>(ws + L.lj) : nullptr;
   auto *box = reinterpret_cast<PairBox<T> *>(ws + L.box);
   a.atoms = atoms;
   a.lj = lj;
@@ -575,7 +604,7 @@ int run_pairs(const PairCall &c, cudaStream_t s) {
   };
   int st = launch_k(false, pair_prep_kernel<T>, blocks(std::max(c.natoms, nacc2)), kPairBlock, 0, s, c.natoms,
                     static_cast<const T *>(c.x), c.cm != C_NONE ? static_cast<const T *>(c.q) : nullptr,
-                    c.lm == L_TYPE ? c.types : nullptr, a.sig, a.eps, static_cast<const T *>(c.box), atoms, lj, box,
+                    c.lm == L_TYPE ? c.types : nullptr, a.sig, a.eps, static_cast<const T *>(c.box), atoms, wide, lj, box,
                     reinterpret_cast<ulonglong2 *>(ws), nacc2, a.ticket);
   if (st != TFF_OK) return st;
   const int64_t total = c.npairs + (c.cm == C_EWALD ? c.nexcl : 0);
