@@ -337,15 +337,12 @@ int batch_enqueue(tff_batch b, int kclass, const T *x, const T *boxes, const T *
   cluster_bounds_kernel<T><<<(int)std::max<int64_t>(1, std::min<int64_t>(L.supers, 2 * sms)), kWarp * kSuper, 0, s>>>(cd);
   TFF_LAUNCHED();
   const int nb_cl = (int)std::max<int64_t>(1, std::min<int64_t>((L.clusters + 3) / 4, sms * 16));
-  cluster_neighbors_kernel<T><<<nb_cl, 128, 0, s>>>(cd, b->desc.cutoff, kHalfLists<T>);
-  TFF_LAUNCHED();
   auto *lj = reinterpret_cast<typename V2<T>::type *>(w + L.lj);
   int *exslot = reinterpret_cast<int *>(w + L.exslot);
-  {
-    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((slots_cap + 255) / 256, sms * 8));
-    sorted_params_kernel<T><<<nb, 256, 0, s>>>(cd, sigma, eps, excl, lj, exslot);
-    TFF_LAUNCHED();
-  }
+  cluster_neighbors_kernel<T, false><<<nb_cl, 128, 0, s>>>(cd, b->desc.cutoff, kHalfLists<T>, SlotParams<T>{}, nb_cl);
+  TFF_LAUNCHED();
+  if (const int st = launch_slot_params<T>(false, cd, SlotParams<T>{sigma, eps, excl, lj, exslot}, slots_cap, s); st != TFF_OK)
+    return st;
   S *e_tile = reinterpret_cast<S *>(w + L.e_tile);
   {
     TileArgs<T> A;

@@ -131,11 +131,18 @@ int system_eval_impl(tff_system sys, const T *x, const T *box, double *energy, T
 
   // --- real space on the caller stream
   ClusterData<T> cd = cluster_data<T>(sys->cl, sys->cl_ws);
-  // the real-space chain (cluster build, sorted parameters, tile kernel) is one run of
+  S *gx = static_cast<S *>(sys->acc);
+  S *gq = gx + 3 * sys->cl.npad;
+  auto *lj = static_cast<typename V2<T>::type *>(sys->lj);
+  SlotParams<T> params{static_cast<const T *>(sys->sigma), static_cast<const T *>(sys->eps), sys->excl, lj,
+                       sys->exslot};
+  params.gx = gx;
+  params.gq = gq;
+  // the real-space chain (cluster build with the sorted parameters, tile kernel) is one run of
   // programmatic dependent launches unless stage events sit between its kernels
   const bool pdl = ev == nullptr;
   st = build_clusters<T>(sys->cl, cd, sys->cl_ws, x, static_cast<const T *>(sys->q), box, sys->desc.cutoff,
-                         kHalfLists<T>, s, sys->scratch, 8 * sizeof(double), pdl);
+                         kHalfLists<T>, s, sys->scratch, 8 * sizeof(double), pdl, params);
   if (st != TFF_OK) return st;
   if ((st = mark(1, s)) != TFF_OK) return st;
   if (use_pme) {
@@ -150,19 +157,12 @@ int system_eval_impl(tff_system sys, const T *x, const T *box, double *energy, T
     TFF_CUDA(cudaEventRecord(sys->join_ev, ps));
     e_pme = reinterpret_cast<const double *>(pw + sys->pl.energies);
   }
-  S *gx = static_cast<S *>(sys->acc);
-  S *gq = gx + 3 * sys->cl.npad;
-  auto *lj = static_cast<typename V2<T>::type *>(sys->lj);
   if (n > 0) {
-    // sorted parameters; also zeroes the accumulators
-    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((sys->cl.npad + 255) / 256, sms * 8));
-    st = launch_k(pdl, sorted_params_kernel<T>, nb, 256, 0, s, cd, static_cast<const T *>(sys->sigma),
-                  static_cast<const T *>(sys->eps), static_cast<const int *>(sys->excl), lj, sys->exslot,
-                  static_cast<const T *>(nullptr), static_cast<typename V4<T>::type *>(nullptr), gx, gq,
-                  static_cast<S *>(nullptr));
-    if (st != TFF_OK) return st;
+    if (!build_writes_slots(sys->cl) && (st = launch_slot_params<T>(pdl, cd, params, sys->cl.npad, s)) != TFF_OK)
+      return st;
     TileArgs<T> A;
     A.cl = cd;
+    if (build_writes_slots(sys->cl)) A.cl.items = nullptr;  // not filled
     A.lj = lj;
     A.exslot = sys->exslot;
     A.gx = gx;
@@ -288,23 +288,30 @@ int system_grad_impl(tff_system sys, const T *x, const T *box, const T *dir, dou
     TFF_CUDA(cudaEventRecord(sys->join_ev, ps));
   }
   ClusterData<T> cd = cluster_data<T>(sys->cl, sys->cl_ws);
-  // one run of programmatic dependent launches, as in the energy evaluation; the build zeroes the
-  // energy accumulators, the sorted parameters the per-slot ones
-  int st = build_clusters<T>(sys->cl, cd, sys->cl_ws, x, static_cast<const T *>(sys->q), box, sys->desc.cutoff, 0, s,
-                             sys->scratch, 8 * sizeof(double), true);
-  if (st != TFF_OK) return st;
   S *acc = static_cast<S *>(sys->acc);
   const int64_t np = sys->cl.npad;
   auto *lj = static_cast<typename V2<T>::type *>(sys->lj);
   auto *dsorted = static_cast<typename V4<T>::type *>(sys->dir_sorted);
+  SlotParams<T> params{static_cast<const T *>(sys->sigma), static_cast<const T *>(sys->eps), sys->excl, lj,
+                       sys->exslot};
+  if (MODE == 2) {
+    params.dir = dir;
+    params.dir_sorted = dsorted;
+  }
+  params.gx = acc;
+  params.gq = acc + 3 * np;
+  params.gp = acc + 4 * np;
+  // one run of programmatic dependent launches, as in the energy evaluation; the build zeroes the
+  // energy accumulators and the per-slot ones
+  int st = build_clusters<T>(sys->cl, cd, sys->cl_ws, x, static_cast<const T *>(sys->q), box, sys->desc.cutoff, 0, s,
+                             sys->scratch, 8 * sizeof(double), true, params);
+  if (st != TFF_OK) return st;
   if (n > 0) {
-    const int nb = (int)std::max<int64_t>(1, std::min<int64_t>((np + 255) / 256, sms * 8));
-    st = launch_k(true, sorted_params_kernel<T>, nb, 256, 0, s, cd, static_cast<const T *>(sys->sigma),
-                  static_cast<const T *>(sys->eps), static_cast<const int *>(sys->excl), lj, sys->exslot,
-                  MODE == 2 ? dir : static_cast<const T *>(nullptr), dsorted, acc, acc + 3 * np, acc + 4 * np);
-    if (st != TFF_OK) return st;
+    if (!build_writes_slots(sys->cl) && (st = launch_slot_params<T>(true, cd, params, sys->cl.npad, s)) != TFF_OK)
+      return st;
     TileArgs<T> A;
     A.cl = cd;
+    if (build_writes_slots(sys->cl)) A.cl.items = nullptr;  // not filled
     A.lj = lj;
     A.exslot = sys->exslot;
     A.gx = acc;
@@ -789,9 +796,9 @@ int tff_system_hvp(tff_system sys, const void *coords, const void *box, const vo
 
 int tff_system_kernel_launches(tff_system sys) {
   if (!sys) return 0;
-  // cluster build 7 (1 for a small system) + sorted params 1 + tile 1 + finalize 1; PME: spread, solve,
-  // gather. The solve is three plane kernels, or [to_real] and the convolution between cuFFT's
-  int k = small_build(sys->cl) ? 4 : 10;
+  // cluster build 7 (1 for a small system) + slot parameters of a large one + tile 1 + finalize 1; PME:
+  // spread, solve, gather. The solve is three plane kernels, or [to_real] and the convolution between cuFFT's
+  int k = small_build(sys->cl) ? 3 : build_writes_slots(sys->cl) ? 9 : 10;
   if (sys->pme) k += sys->pme->impl.planes ? 5 : sys->desc.dtype == TFF_F32 ? 4 : 3;
   return k;
 }

@@ -235,16 +235,7 @@ __global__ void __launch_bounds__(kEmitBlock) cell_emit_kernel(ClusterData<T> d,
   const int ncl = (int)d.nclusters;
   const int nitems = d.itemoff[ncl];
   for (int item = blockIdx.x * kEmitWarps + w; item < nitems; item += gridDim.x * kEmitWarps) {
-    // cluster I with itemoff[I] <= item < itemoff[I + 1]: 32 probes per step
-    int I = 0;
-    for (int len = ncl; len > 1;) {
-      const int step = (len + kWarp - 1) / kWarp;
-      const int at = I + lane * step;
-      const unsigned le = __ballot_sync(kFull, lane * step < len && d.itemoff[at] <= item);
-      const int k = 31 - __clz(le);  // the lowest probe always holds
-      len = min(step, len - k * step);
-      I += k * step;
-    }
+    const int I = item_cluster(d.itemoff, ncl, item);
     const int k0 = item - d.itemoff[I], n = d.itemoff[I + 1] - d.itemoff[I], cnt = d.ncount[I];
     const int64_t si = (int64_t)I * kWarp + lane;
     const int ai = d.sidx[si];

@@ -233,7 +233,7 @@ template <class T> struct PairTileOcc { static constexpr int min_blocks = sizeof
 
 // FP32 only: FP64 real space runs on full lists and tile_kernel (see launch_real_space). ERF: how the
 // FP64 exclusion correction is evaluated (erf_poly.cuh).
-template <class T, int NW, int MIN_BLOCKS, int ERF>
+template <class T, int NW, int MIN_BLOCKS, int ERF, bool TABLE>
 __global__ void __launch_bounds__(NW * 32, MIN_BLOCKS) pair_tile_kernel(TileArgs<T> A, PairConst<T> pc) {
   static_assert(sizeof(T) == 4, "the pair kernel is the FP32 real-space kernel");
   pdl_enter();
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(NW * 32, MIN_BLOCKS) pair_tile_kernel(TileArgs
   const int nitems = cl.itemoff[cl.n_clusters()];
   const int nwarps = gridDim.x * NW;
   for (int it = blockIdx.x * NW + w; it < nitems; it += nwarps) {
-    const int I = cl.items[it];  // owning cluster: itemoff[I] <= it < itemoff[I + 1]
+    const int I = TABLE ? cl.items[it] : item_cluster(cl.itemoff, (int)cl.n_clusters(), it);
     const int isys = cl.system_of(I);
     const double *info = cl.info(isys);
     if (isys != cur_sys) {
@@ -587,11 +587,15 @@ int launch_real_space(bool pdl, int64_t max_items, int sms, cudaStream_t s, cons
       return launch_k(pdl, kernel, nbt, NW * kWarp, 0, s, A, pair_const<T>(A.alpha));
     };
     constexpr int MB = PairTileOcc<T>::min_blocks;
-    switch (erf_range(A.alpha, A.rc)) {
-      case kErfShort: return launch(pair_tile_kernel<T, NW, MB, kErfShort>);
-      case kErfLong: return launch(pair_tile_kernel<T, NW, MB, kErfLong>);
-      default: return launch(pair_tile_kernel<T, NW, MB, kErfLibrary>);
+    const ErfRange range = erf_range(A.alpha, A.rc);
+    if (A.cl.items) {
+      if (range == kErfShort) return launch(pair_tile_kernel<T, NW, MB, kErfShort, true>);
+      if (range == kErfLong) return launch(pair_tile_kernel<T, NW, MB, kErfLong, true>);
+      return launch(pair_tile_kernel<T, NW, MB, kErfLibrary, true>);
     }
+    if (range == kErfShort) return launch(pair_tile_kernel<T, NW, MB, kErfShort, false>);
+    if (range == kErfLong) return launch(pair_tile_kernel<T, NW, MB, kErfLong, false>);
+    return launch(pair_tile_kernel<T, NW, MB, kErfLibrary, false>);
   } else {
     return launch_tile<T, 0>(pdl, max_items, sms, s, A);
   }

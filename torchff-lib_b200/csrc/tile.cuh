@@ -27,7 +27,6 @@
 namespace tff {
 namespace {
 
-constexpr int kMaxExcl = 8;       // excluded partners per atom (self excluded)
 
 // Warps per block of the tile kernel: 4 (FP32) or 2 (FP64) so that the staged tiles fit in
 // 48 KB of static shared memory.
@@ -37,12 +36,6 @@ template <class T, int MODE = 0> struct TileCfg {
   static constexpr int NW = (sizeof(T) == 8 || MODE == 2) ? 2 : 4;
 };
 
-template <class T> struct V2;
-template <> struct V2<float> { using type = float2; };
-struct __align__(16) D2 { double x, y; };
-template <> struct V2<double> { using type = D2; };
-__device__ __forceinline__ float2 make_v2(float a, float b) { return make_float2(a, b); }
-__device__ __forceinline__ D2 make_v2(double a, double b) { return D2{a, b}; }
 
 __device__ __forceinline__ float erf_t(float x) { return erff(x); }
 __device__ __forceinline__ double erf_t(double x) { return erf(x); }
@@ -70,48 +63,6 @@ struct TileArgs {
   typename Acc<T>::S *ga = nullptr;  // MODE 1/2: (npad) d/da_i, a = sqrt(eps)
   const typename V4<T>::type *u = nullptr;  // MODE 2: direction per sorted slot
 };
-
-// LB parameters and excluded-partner slots in sorted order. Partner indices are counted
-// from the first atom of the atom's own system (batch mode), i.e. global for one system.
-// With `dir` (caller order (N,3)) also the direction of a second-derivative pass in
-// sorted order.
-// With `gx` / `gq` also zeroes the tile kernel's accumulators of each slot (3 + 1 values, with
-// `gp` the npad slots of each parameter derivative too).
-// Also fills the tile kernel's item -> cluster table from the item offsets of the
-// neighbour search (the lanes of cluster k write its entries).
-template <class T>
-__global__ void sorted_params_kernel(ClusterData<T> cl, const T *sigma, const T *eps, const int *excl,
-                                     typename V2<T>::type *lj, int *exslot, const T *dir = nullptr,
-                                     typename V4<T>::type *dir_sorted = nullptr, typename Acc<T>::S *gx = nullptr,
-                                     typename Acc<T>::S *gq = nullptr, typename Acc<T>::S *gp = nullptr) {
-  pdl_enter();
-  const int64_t npad = cl.n_pad();
-  for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s < npad; s += (int64_t)gridDim.x * blockDim.x) {
-    if (gx) {
-      gx[3 * s] = 0;
-      gx[3 * s + 1] = 0;
-      gx[3 * s + 2] = 0;
-      gq[s] = 0;
-    }
-    if (gp) gp[s] = gp[npad + s] = 0;
-    {
-      const int64_t k = s / kWarp;
-      const int o = cl.itemoff[k], nk = cl.itemoff[k + 1] - o;
-      for (int j = (int)(s % kWarp); j < nk; j += kWarp) cl.items[o + j] = (int)k;
-    }
-    const int a = cl.sidx[s];
-    if (dir)
-      dir_sorted[s] = a >= 0 ? make_v4(dir[3 * (int64_t)a], dir[3 * (int64_t)a + 1], dir[3 * (int64_t)a + 2], T(0))
-                             : make_v4(T(0), T(0), T(0), T(0));
-    const int64_t base = (cl.sys && a >= 0) ? cl.sys[cl.cl_sys[s / kWarp]].atom_off : 0;
-    lj[s] = a >= 0 ? make_v2(T(0.5) * sigma[a], (T)sqrt((double)eps[a])) : make_v2(T(0), T(0));
-#pragma unroll
-    for (int k = 0; k < kMaxExcl; ++k) {
-      const int p = a >= 0 ? excl[(int64_t)a * kMaxExcl + k] : -1;
-      exslot[s * kMaxExcl + k] = p >= 0 ? cl.inv[base + p] : -1;
-    }
-  }
-}
 
 template <class T>
 __device__ __forceinline__ void pair_min_image(bool ortho, T &dx, T &dy, T &dz, const T *m, const T *inv) {
@@ -163,7 +114,7 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? kTileMi
   const int nitems = cl.itemoff[cl.n_clusters()];
   const int nwarps = gridDim.x * NW;
   for (int it = blockIdx.x * NW + w; it < nitems; it += nwarps) {
-    const int I = cl.items[it];  // owning cluster: itemoff[I] <= it < itemoff[I + 1]
+    const int I = cl.items ? cl.items[it] : item_cluster(cl.itemoff, (int)cl.n_clusters(), it);
     const int isys = cl.system_of(I);
     if (isys != cur_sys) {
       const double *info = cl.info(isys);
