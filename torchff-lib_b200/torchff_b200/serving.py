@@ -103,7 +103,7 @@ class BatchEvaluator:
 
     def graph_launches(self) -> int:
         """Evaluations so far that replayed a captured CUDA graph (evaluate_packed on the
-        same device buffers and DFT size class as the call before captures one)."""
+        same device buffers and transform size class as the call before captures one)."""
         return int(lib.tff_batch_graph_launches(self._h))
 
     def pack(self, systems: list[SystemSpec]) -> dict:
