@@ -1,21 +1,33 @@
-// erf(sqrt(y)) / sqrt(y) and its first two derivatives for FP64 Ewald terms.
+// FP64 Ewald terms by polynomials: erfcx for pairs, erf(sqrt(y)) / sqrt(y) and its first two
+// derivatives for excluded pairs.
 //
-// H(y) = erf(sqrt(y)) / sqrt(y) = 2/sqrt(pi) sum_n (-y)^n / (n! (2n + 1)) is entire, so on a bounded
-// range of y = (alpha r)^2 - the cutoff bounds it - a polynomial in y gives it to FP64 rounding, and
-// the screened Coulomb terms follow without erfc, exp or a branch:
+// Pairs: on a bounded range of u = alpha r - the cutoff bounds it - erfcx(u) = exp(u^2) erfc(u) lies
+// between 0.15 and 1 and a polynomial in u gives it to FP64 rounding. With X = exp(-(alpha r)^2) and
+// t = 2 alpha / sqrt(pi) the screened Coulomb terms are sums of positive parts:
 //
-//   erfc(alpha r) / r                = 1/r - alpha H
-//   -(1/r) d/dr [erfc(alpha r) / r]  = 1/r^3 + 2 alpha^3 H'
-//   (1/r) d/dr of (1/r) d/dr [...]   = 3/r^5 - 4 alpha^5 H''
+//   f = erfc(alpha r) / r  = X erfcx / r
+//   g = -(1/r) df/dr       = (f + t X) / r^2
+//   h = -(1/r) dg/dr       = (3 g + 2 alpha^2 t X) / r^2
 //
-// (exclusion corrections are the H parts alone). The subtraction from 1/r leaves an absolute error
-// of about 1e-16 / r, the rounding of the unscreened term. Coefficients: Chebyshev interpolation of
-// the series on [0, Y] in 60 digits, turned into powers of z = 2 y / Y - 1 in [-1, 1] (largest
-// deviation below 2e-17 of H(0), H'(0), H''(0); the powers' magnitudes sum to that value, so Horner's
-// rule loses nothing). They sit in constant memory and are operands of the multiply-adds.
+// The argument of X is one product of r^2, so its rounding error is what the terms' relative error
+// grows from, 6e-16 to 2.7e-15 at u = 3.7 (with erfc(u) and exp(-u^2) of a rounded u: 1.1e-14).
 //
-// What bounds the FP64 real-space kernels is the FP64 pipe (half the FP32 rate): erfc, exp and their
-// branches were most of their operations. FP64 evaluation of 3000 waters 198 -> 145 us.
+// Excluded pairs: H(y) = erf(sqrt(y)) / sqrt(y) = 2/sqrt(pi) sum_n (-y)^n / (n! (2n + 1)) is entire, and
+//
+//   -erf(alpha r) / r and its g and h  =  -alpha H,  2 alpha^3 H',  -4 alpha^5 H''
+//
+// have no cancellation at short range, where excluded pairs are. H'' falls off as y^-5/2, below the
+// rounding of its first coefficients: beyond y = 6, h is taken from g as above. Relative errors below
+// 1.4e-15. (The same functions as differences, 1/r - alpha H for pairs, would leave the rounding of
+// 1/r: 1e-9 of erfc(alpha r) / r at u = 3.7.)
+//
+// Coefficients: Chebyshev interpolation of the functions on the range in 60 digits, turned into
+// powers of z in [-1, 1] (z = 2 u / U - 1, 2 y / Y - 1). Largest deviations: 5e-17 of erfcx, 2e-17 of
+// H(0), H'(0), H''(0); the powers' magnitudes sum to the function's value at 0, so Horner's rule loses
+// nothing. They sit in constant memory and are operands of the multiply-adds.
+//
+// Bound by latency and the FP64 pipe together: erfc with its branches was most of the operations of the
+// FP64 real-space kernels. FP64 evaluation of 3000 waters with erfc and exp 198 us, with this 141 us.
 #pragma once
 
 #include "tff_common.cuh"
@@ -29,6 +41,7 @@ enum ErfRange { kErfLibrary = 0, kErfShort, kErfLong };
 
 inline ErfRange erf_range(double alpha, double rc) {
   const double y = alpha * alpha * rc * rc;
+  if (!(alpha >= 0.0)) return kErfLibrary;
   return y <= 7.0 ? kErfShort : y <= 13.5 ? kErfLong : kErfLibrary;
 }
 
@@ -76,9 +89,34 @@ __constant__ double kErfCoefLong[3][27] = {
      3.8592606978322097887e-9, -1.627100033618517895e-9, 3.9291631250974622532e-10},
 };
 
-template <int RANGE> struct ErfDegree;  // of H, H', H''
-template <> struct ErfDegree<kErfShort> { static constexpr int n[3] = {20, 20, 21}; static constexpr double y = 7.0; };
-template <> struct ErfDegree<kErfLong> { static constexpr int n[3] = {25, 26, 26}; static constexpr double y = 13.5; };
+// erfcx(u) in powers of 2 u / U - 1, U^2 = 7 and 13.5.
+__constant__ double kErfcxCoefShort[25] = {
+    0.3531532283889421921, -0.25666903099916359337, 0.16884734543211193357, -0.10245863316159168163,
+    0.05809012323674185174, -0.031057956946421562583, 0.015768763668503901146, -0.0076445966529360104245,
+    0.0035543230794671415144, -0.0015906618329095274079, 0.00068728136450534367756,
+    -0.00028743979770065836015, 0.00011662078099687772321, -0.000045987926838163079709,
+    0.000017657237930247742722, -6.6144335323863888947e-6, 2.4176165993335347268e-6,
+    -8.5824052991708958034e-7, 3.0039743907920067315e-7, -1.084835386026760684e-7, 3.6247527418719507079e-8,
+    -8.4335147430632918725e-9, 2.8038293758428327001e-9, -2.1707353931562656211e-9, 6.659930472064703272e-10};
+__constant__ double kErfcxCoefLong[29] = {
+    0.27397089384189582418, -0.22366136339521592096, 0.16979466525754414481, -0.12120007080978147654,
+    0.082003378130640144243, -0.052915535116002857712, 0.032723823390237260079, -0.019470579180527974838,
+    0.011182424821373752461, -0.0062161155878497081127, 0.0033522585481755089156, -0.0017573680810650316636,
+    0.00089712702790560685137, -0.00044665777265440253939, 0.00021718571179207336212,
+    -0.00010328123783356989007, 0.000048067829252725247285, -0.000021880191198089287871,
+    9.789641006485781542e-6, -4.3646411342156628541e-6, 1.8781603296814997535e-6, -7.1973030617069291164e-7,
+    3.0365900537636943908e-7, -1.8515428733865061121e-7, 7.2810666586545844097e-8, 2.5495578952404890615e-9,
+    -3.339947450605960353e-10, -9.5918066883621116037e-9, 3.5640640174143862978e-9};
+
+template <int RANGE> struct ErfDegree;  // of H, H', H'', of erfcx; ends of the range in y and u
+template <> struct ErfDegree<kErfShort> {
+  static constexpr int n[3] = {20, 20, 21}, x = 24;
+  static constexpr double y = 7.0, u = 2.6457513110645905905;
+};
+template <> struct ErfDegree<kErfLong> {
+  static constexpr int n[3] = {25, 26, 26}, x = 28;
+  static constexpr double y = 13.5, u = 3.6742346141747672955;
+};
 
 // K-th derivative of H at z = 2 y / Y - 1.
 template <int RANGE, int K>
@@ -98,32 +136,50 @@ __device__ __forceinline__ double rcp_newton(double x, double y) {
   return fma(v, fma(-x, v, 1.0), v);
 }
 
-// Screened Coulomb of one pair: f = erfc(alpha r) / r, g = -(1/r) df/dr, second() = -(1/r) dg/dr;
-// excluded pairs: the same of -erf(alpha r) / r.
+template <int RANGE>
+__device__ __forceinline__ double erfcx_poly(double z) {
+  constexpr int n = ErfDegree<RANGE>::x;
+  static_assert(n % 2 == 0, "the even chain starts at the highest power");
+  const auto c = [](int i) { return RANGE == kErfShort ? kErfcxCoefShort[i] : kErfcxCoefLong[i]; };
+  // even and odd powers apart: two chains half as long (143.8 -> 141.4 us of that evaluation)
+  const double w = z * z;
+  double even = c(n), odd = c(n - 1);
+#pragma unroll
+  for (int i = n - 2; i >= 0; i -= 2) even = fma(even, w, c(i));
+#pragma unroll
+  for (int i = n - 3; i >= 1; i -= 2) odd = fma(odd, w, c(i));
+  return fma(odd, z, even);
+}
+
+// Terms f, g, h of one pair (see above); excluded pairs: of -erf(alpha r) / r.
 template <int RANGE>
 struct EwaldPoly {
-  double zs, a, a3, a5;  // 2 alpha^2 / Y, alpha, 2 alpha^3, 4 alpha^5
+  double a, y, u, t, a3;  // alpha, alpha^2, 2 alpha / U, 2 alpha / sqrt(pi), 2 alpha^3
   __device__ __forceinline__ explicit EwaldPoly(double alpha) {
     a = alpha;
-    zs = alpha * alpha * (2.0 / ErfDegree<RANGE>::y);
-    a3 = 2.0 * alpha * alpha * alpha;
-    a5 = 2.0 * a3 * alpha * alpha;
+    y = alpha * alpha;
+    u = alpha * (2.0 / ErfDegree<RANGE>::u);
+    t = 2.0 * alpha / 1.7724538509055160273;
+    a3 = 2.0 * alpha * y;
   }
-  __device__ __forceinline__ void eval(double r2, double rinv, double rinv2, double &f, double &g) const {
-    const double z = fma(r2, zs, -1.0);
-    f = fma(-a, erf_poly<RANGE, 0>(z), rinv);
-    g = fma(a3, erf_poly<RANGE, 1>(z), rinv * rinv2);
+  // tx: t X
+  __device__ __forceinline__ void eval(double r2, double rinv, double rinv2, double &f, double &g, double &tx) const {
+    const double x = exp(-y * r2);
+    f = x * erfcx_poly<RANGE>(fma(r2 * rinv, u, -1.0)) * rinv;
+    tx = t * x;
+    g = (f + tx) * rinv2;
   }
-  __device__ __forceinline__ double second(double r2, double rinv, double rinv2) const {
-    return fma(-a5, erf_poly<RANGE, 2>(fma(r2, zs, -1.0)), 3.0 * rinv * rinv2 * rinv2);
+  __device__ __forceinline__ double second(double rinv2, double g, double tx) const {
+    return fma(2.0 * y, tx, 3.0 * g) * rinv2;
   }
+  __device__ __forceinline__ double z(double r2) const { return fma(r2, y * (2.0 / ErfDegree<RANGE>::y), -1.0); }
   __device__ __forceinline__ void excluded(double r2, double &f, double &g) const {
-    const double z = fma(r2, zs, -1.0);
-    f = -a * erf_poly<RANGE, 0>(z);
-    g = a3 * erf_poly<RANGE, 1>(z);
+    f = -a * erf_poly<RANGE, 0>(z(r2));
+    g = a3 * erf_poly<RANGE, 1>(z(r2));
   }
-  __device__ __forceinline__ double excluded_second(double r2) const {
-    return -a5 * erf_poly<RANGE, 2>(fma(r2, zs, -1.0));
+  __device__ __forceinline__ double excluded_second(double r2, double g) const {
+    if (y * r2 > 6.0) return second(1.0 / r2, g, t * exp(-y * r2));
+    return -2.0 * a3 * y * erf_poly<RANGE, 2>(z(r2));
   }
 };
 

@@ -308,11 +308,11 @@ __global__ void __launch_bounds__(kPairBlock, sizeof(T) == 4 ? 4 : 3) pair_kerne
               f = rinv;
               dfdr_r = -rinv2 * rinv;
             } else if constexpr (ERF != kErfLibrary) {
-              T g;
+              T g, tx;
               if (is_excl)
                 ewald.excluded(r2, f, g);
               else
-                ewald.eval(r2, rinv, rinv2, f, g);
+                ewald.eval(r2, rinv, rinv2, f, g, tx);
               dfdr_r = -g;
             } else {
               const T r = r2 * rinv;

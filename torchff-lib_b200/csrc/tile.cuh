@@ -322,8 +322,9 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? kTileMi
           if constexpr (ERF != kErfLibrary) {
             rinv = rsqrt_t(r2);
             rinv2 = rcp_newton(r2, rinv);
-            ewald.eval(r2, rinv, rinv2, f, g);
-            if constexpr (MODE == 2) h = ewald.second(r2, rinv, rinv2);
+            T tx;
+            ewald.eval(r2, rinv, rinv2, f, g, tx);
+            if constexpr (MODE == 2) h = ewald.second(rinv2, g, tx);
           } else {
             rinv = rsqrt_t(r2);
             rinv2 = rinv * rinv;
@@ -392,7 +393,8 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? kTileMi
           if constexpr (ERF != kErfLibrary) {
             rinv = rsqrt_t(r2);
             rinv2 = rcp_newton(r2, rinv);
-            ewald.eval(r2, rinv, rinv2, f, g);
+            T tx;
+            ewald.eval(r2, rinv, rinv2, f, g, tx);
           } else {
             rinv = rsqrt_t(r2);
             rinv2 = rinv * rinv;
@@ -438,7 +440,7 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? kTileMi
         T f, g, h = T(0);
         if constexpr (ERF != kErfLibrary) {
           ewald.excluded(r2, f, g);
-          if constexpr (MODE == 2) h = ewald.excluded_second(r2);
+          if constexpr (MODE == 2) h = ewald.excluded_second(r2, g);
         } else {
           const T rinv = rsqrt_t(r2);
           const T u = alpha * (r2 * rinv);
