@@ -1007,7 +1007,7 @@ __global__ void cluster_neighbors_kernel(ClusterData<T> d, double rc, int half, 
 }
 
 // Steps 1-6 of a small system in one launch of one block: a thread per atom, a warp per cluster.
-// Up to kSmallAtoms atoms (32 clusters, one super-cluster) the seven launches of the general build
+// Up to kSmallAtoms atoms (32 clusters, one super-cluster) the six launches of the general build
 // are latency from end to end (648 atoms: 34 us of kernels, 41 with the slot parameters; this one 8.8
 // and 13.7 us); the sort order, boxes, lists and work items are the same.
 constexpr int kSmallAtoms = 1024;
@@ -1156,6 +1156,13 @@ inline bool small_build(const ClusterLayout &L) {
 
 // Whether build_clusters writes the slot parameters it is given, or a launch_slot_params must follow.
 inline bool build_writes_slots(const ClusterLayout &L) { return small_build(L) || slots_beside_search(L.nclusters); }
+
+// Kernels build_clusters launches: without atoms the box alone; up to kFusedScanMaxKeys keys the scan
+// rides in the key kernel.
+inline int build_launches(const ClusterLayout &L) {
+  if (small_build(L) || L.natoms == 0) return 1;
+  return L.nkeys <= kFusedScanMaxKeys ? 6 : 7;
+}
 
 // Host driver for steps 1-6 on `stream`. `zero` (`zero_bytes`, a multiple of 8) is cleared
 // on the way. With `pdl` every kernel after the first is a programmatic dependent launch.

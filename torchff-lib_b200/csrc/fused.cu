@@ -796,9 +796,14 @@ int tff_system_hvp(tff_system sys, const void *coords, const void *box, const vo
 
 int tff_system_kernel_launches(tff_system sys) {
   if (!sys) return 0;
-  // cluster build 7 (1 for a small system) + slot parameters of a large one + tile 1 + finalize 1; PME:
-  // spread, solve, gather. The solve is three plane kernels, or [to_real] and the convolution between cuFFT's
-  int k = small_build(sys->cl) ? 3 : build_writes_slots(sys->cl) ? 9 : 10;
+  const bool atoms = sys->desc.natoms > 0;
+  // cluster build and finalize; with atoms the real-space kernel, the slot parameters of a large system, the
+  // bonded terms, and of PME: spread, solve, gather. The solve is three plane kernels, or [to_real] and the
+  // convolution between cuFFT's
+  int k = build_launches(sys->cl) + 1;
+  if (!atoms) return k;
+  k += build_writes_slots(sys->cl) ? 1 : 2;
+  if (sys->has_bonded()) ++k;
   if (sys->pme) k += sys->pme->impl.planes ? 5 : sys->desc.dtype == TFF_F32 ? 4 : 3;
   return k;
 }
