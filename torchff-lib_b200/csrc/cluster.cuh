@@ -87,6 +87,7 @@ struct ClusterLayout {
   int nc = 1, bits = 0;
   int64_t nkeys = 1, natoms = 0, nclusters = 0, npad = 0, nsuper = 0;
   int cap = 0;
+  bool has_items = false;
   size_t keys, hist, fill, status, tmp, sidx, inv, pos, frac, bc, bh, sbc, sbh, nbr, ncount, itemoff, items, boxinfo;
   size_t zero_off, zero_bytes, bytes;
 };
@@ -106,8 +107,10 @@ inline void cell_grid(int64_t natoms, double atoms_per_cell, int &nc, int &bits)
   while ((1 << bits) < nc) ++bits;
 }
 
-inline ClusterLayout cluster_layout(int dtype, int64_t natoms, int cap) {
+// `items`: with room for the cluster of each work item (see slot_params_kernel).
+inline ClusterLayout cluster_layout(int dtype, int64_t natoms, int cap, bool items) {
   ClusterLayout L;
+  L.has_items = items;
   L.natoms = natoms;
   int nc, bits;
   cell_grid(natoms, 8.0, nc, bits);
@@ -139,7 +142,7 @@ inline ClusterLayout cluster_layout(int dtype, int64_t natoms, int cap) {
   L.nbr = (c.off + 255) & ~size_t(255); c.take<int>((size_t)L.nclusters * cap);
   L.ncount = (c.off + 255) & ~size_t(255); c.take<int>(L.nclusters);
   L.itemoff = (c.off + 255) & ~size_t(255); c.take<int>(L.nclusters + 1);
-  L.items = (c.off + 255) & ~size_t(255); c.take<int>((size_t)item_capacity(L.nclusters, cap));
+  L.items = (c.off + 255) & ~size_t(255); c.take<int>(items ? (size_t)item_capacity(L.nclusters, cap) : 0);
   L.boxinfo = (c.off + 255) & ~size_t(255); c.take<double>(32);
   L.bytes = c.bytes();
   return L;
@@ -218,7 +221,7 @@ inline ClusterData<T> cluster_data(const ClusterLayout &L, void *ws) {
   d.nbr = reinterpret_cast<int *>(b + L.nbr);
   d.ncount = reinterpret_cast<int *>(b + L.ncount);
   d.itemoff = reinterpret_cast<int *>(b + L.itemoff);
-  d.items = reinterpret_cast<int *>(b + L.items);
+  d.items = L.has_items ? reinterpret_cast<int *>(b + L.items) : nullptr;
   d.pos = reinterpret_cast<V *>(b + L.pos);
   d.frac = reinterpret_cast<V *>(b + L.frac);
   d.bc = reinterpret_cast<V *>(b + L.bc);

@@ -36,7 +36,7 @@ struct CpLayout {
 
 inline CpLayout cp_layout(int dtype, int64_t natoms, int cap) {
   CpLayout L;
-  L.cl = cluster_layout(dtype, natoms, cap);
+  L.cl = cluster_layout(dtype, natoms, cap, false);
   Carver c(nullptr);
   c.off = L.cl.bytes;
   L.exset = (c.off + 255) & ~size_t(255); c.take<int>((size_t)L.cl.nclusters * kMaxExclClusters);

@@ -405,7 +405,7 @@ int tff_system_create(const tff_system_desc *desc, const double *charges, const 
   const int64_t ncl = (n + kWarp - 1) / kWarp;
   sys->cap = desc->max_cluster_neighbors > 0 ? desc->max_cluster_neighbors
                                              : (int)std::max<int64_t>(1, std::min<int64_t>(ncl, 1024));
-  sys->cl = cluster_layout(desc->dtype, n, sys->cap);
+  sys->cl = cluster_layout(desc->dtype, n, sys->cap, true);
   const size_t ts = desc->dtype == TFF_F64 ? 8 : 4;
 #define TFF_ALLOC(ptr, bytes)                                              \
   do {                                                                     \

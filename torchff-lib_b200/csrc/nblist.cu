@@ -369,7 +369,7 @@ int cell_list_impl(int64_t natoms, const T *x, const T *box, double cutoff, cons
                    size_t ws_bytes, cudaStream_t s) {
   const int dtype = sizeof(T) == 8 ? TFF_F64 : TFF_F32;
   const int64_t ncl = (natoms + kWarp - 1) / kWarp;
-  ClusterLayout L = cluster_layout(dtype, natoms, default_cluster_cap(ncl, ccap));
+  ClusterLayout L = cluster_layout(dtype, natoms, default_cluster_cap(ncl, ccap), false);
   if (ws == nullptr || ws_bytes < L.bytes) {
     set_error("workspace too small: need %zu bytes, got %zu", L.bytes, ws_bytes);
     return TFF_ERR_WORKSPACE;
@@ -420,7 +420,7 @@ int tff_nblist_nsquared(int dtype, int64_t natoms, const void *coords, const voi
 
 size_t tff_nblist_cell_list_workspace_bytes(int dtype, int64_t natoms, int max_cluster_neighbors) {
   const int64_t ncl = (natoms + kWarp - 1) / kWarp;
-  return cluster_layout(dtype, natoms, default_cluster_cap(ncl, max_cluster_neighbors)).bytes;
+  return cluster_layout(dtype, natoms, default_cluster_cap(ncl, max_cluster_neighbors), false).bytes;
 }
 
 int tff_nblist_cell_list(int dtype, int64_t natoms, const void *coords, const void *box, double cutoff,

@@ -4,9 +4,9 @@
 // compute_multipolar_energy_from_atom_pairs.
 //
 // A call is three launches: pair_prep_kernel clears the accumulators and packs every atom's
-// operands into one 16-byte (FP64: 32-byte) record, pair_kernel evaluates one pair per lane,
-// pair_finish_kernel converts the accumulators into the caller's arrays. The work partition -
-// and with it every summation order - depends on the sizes alone.
+// operands into one 16-byte (FP64: 32-byte) record where the workspace has room for them, pair_kernel
+// evaluates one pair per lane, pair_finish_kernel converts the accumulators into the caller's arrays.
+// The work partition - and with it every summation order - depends on the sizes alone.
 // Energies: per-thread FP64, fixed-order block and grid reduction. Gradients: int64
 // fixed-point atomics in mixed precision (order-independent, bit-reproducible), FP64
 // atomics in FP64 mode.
@@ -43,14 +43,17 @@ struct PairBox {
 template <class T>
 struct PairArgs {
   const typename V4<T>::type *atoms;    // (x, y, z, charge); L_TYPE: the type index in the last word.
-                                        // FP32 L_ATOM: two per atom, the second (sigma, epsilon, 0, 0)
+                                        // FP32 L_ATOM: two per atom, the second (sigma, epsilon, 0, 0).
+                                        // NULL: no records, the caller's arrays below are read
   const typename LjRec<T>::type *lj;    // FP64 L_ATOM: (sigma, epsilon)
   const PairBox<T> *box;                // NULL: open boundaries
   const int64_t *pairs;
   int64_t npairs;
   const int64_t *excl;
   int64_t nexcl;
-  const T *sig, *eps;                   // L_PAIR: per pair; L_TYPE: tables
+  const T *x, *q;
+  const int64_t *types;
+  const T *sig, *eps;                   // L_ATOM: per atom; L_PAIR: per pair; L_TYPE: tables
   int64_t ntypes;
   double k, rc, alpha;
   typename Acc<T>::S *acc;              // (natoms, 4): dE/dx, dE/dy, dE/dz, dE/dq; NULL: none of them
@@ -70,7 +73,7 @@ __device__ __forceinline__ double type_bits(double, int t) { return (double)t; }
 __device__ __forceinline__ int bits_type(float w) { return __float_as_int(w); }
 __device__ __forceinline__ int bits_type(double w) { return (int)w; }
 
-// Clears the accumulators and the reduction ticket, packs the atom records and the box.
+// Clears the accumulators and the reduction ticket, packs the records of n atoms (0: none) and the box.
 template <class T>
 __global__ void __launch_bounds__(kPairBlock) pair_prep_kernel(int64_t n, const T *x, const T *q, const int64_t *types,
                                                                const T *sig, const T *eps, const T *box,
@@ -142,10 +145,17 @@ __device__ __forceinline__ double sqrt_t(double x) { return sqrt(x); }
 template <class T, int LM> constexpr bool kWideRec = sizeof(T) == 4 && LM == L_ATOM;
 
 // Record of atom i; `lj` only for L_ATOM.
-template <class T, int LM>
+template <class T, int LM, bool RECORDS>
 __device__ __forceinline__ void load_atom(const PairArgs<T> &a, unsigned i, typename V4<T>::type &r,
                                           typename LjRec<T>::type &lj) {
-  if constexpr (kWideRec<T, LM>) {
+  if constexpr (!RECORDS) {
+    const T w = a.q ? a.q[i] : (a.types ? type_bits(T(0), (int)a.types[i]) : T(0));
+    r = make_v4(a.x[3 * (int64_t)i], a.x[3 * (int64_t)i + 1], a.x[3 * (int64_t)i + 2], w);
+    if (LM == L_ATOM) {
+      lj.x = a.sig[i];
+      lj.y = a.eps[i];
+    }
+  } else if constexpr (kWideRec<T, LM>) {
     float u, v;
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w), "=f"(lj.x), "=f"(lj.y), "=f"(u), "=f"(v)
@@ -187,8 +197,8 @@ constexpr int kStagedRows = kWarp * kMaxPairIters + kWarp * kMaxPairIters / 8;
 // One atomic per value, eight memory clears and conversions per call before: a call over 20.8 M
 // rows (99,000 atoms, FP32) 1,015 -> 515 us, 1.9 M rows of LJ and Ewald (9,000 atoms) 115 and
 // 122 -> 42 and 60 us.
-// ERF (FP64 Ewald): how erfc is evaluated (erf_poly.cuh).
-template <class T, int CM, int LM, int ERF>
+// ERF (FP64 Ewald): how erfc is evaluated (erf_poly.cuh). RECORDS: operands from the packed records.
+template <class T, int CM, int LM, int ERF, bool RECORDS>
 __global__ void __launch_bounds__(kPairBlock, sizeof(T) == 4 ? 4 : 3) pair_kernel(PairArgs<T> a) {
   pdl_enter();
   using A = Acc<T>;
@@ -273,8 +283,8 @@ __global__ void __launch_bounds__(kPairBlock, sizeof(T) == 4 ? 4 : 3) pair_kerne
       if (in) {
         typename V4<T>::type pi, pj;
         typename LjRec<T>::type li{}, lj{};
-        load_atom<T, LM>(a, i, pi, li);
-        load_atom<T, LM>(a, j, pj, lj);
+        load_atom<T, LM, RECORDS>(a, i, pi, li);
+        load_atom<T, LM, RECORDS>(a, j, pj, lj);
         T dx = pi.x - pj.x;
         T dy = pi.y - pj.y;
         T dz = pi.z - pj.z;
@@ -472,25 +482,41 @@ __global__ void __launch_bounds__(kPairBlock) pair_finish_kernel(PairOut<T> a) {
 constexpr size_t kWsAlign = 256;
 
 struct PairLayout {
-  size_t acc, acc_lj, gs_tab, ge_tab;  // accumulators, from offset 0
+  size_t acc, acc_lj, gs_tab, ge_tab, acc_end;  // accumulators, from offset 0
   size_t atoms, lj, box, partials, ticket, energy, bytes;
 };
 
 // Accumulators: 4 per atom (dE/dx, dE/dq), then 2 per atom (dE/dsigma, dE/depsilon) or the type
-// tables'; both accumulator types are 8 bytes.
-PairLayout pair_layout(int dtype, int64_t natoms, int64_t ntypes) {
-  const size_t ts = dtype == TFF_F64 ? 8 : 4;
+// tables'; both accumulator types are 8 bytes. Without records the layout takes the 48 bytes per atom
+// (6 accumulators) and 64.5 KiB that callers of earlier versions of the library reserve: a smaller
+// workspace than tff_pairs_workspace_bytes names is then still enough, and the kernel reads the caller's
+// arrays (the same results; 20.9 M rows over 99,000 atoms with all gradients, FP32: 732 us, with records 687).
+PairLayout pair_layout(int dtype, int64_t natoms, int64_t ntypes, bool records) {
+  const size_t ts = dtype == TFF_F64 ? 8 : 4, tab = (size_t)(ntypes * ntypes) * 8;
   PairLayout L{};
   Carver c(nullptr);
   const auto take = [&c](size_t bytes) {
     c.take<char>(bytes);
     return c.off - bytes;
   };
+  if (!records) {
+    const size_t atom = (size_t)natoms * 8;
+    L.acc_lj = L.gs_tab = 4 * atom;
+    L.ge_tab = L.gs_tab + tab;
+    L.acc_end = 4 * atom + 2 * std::max(atom, tab);
+    take(L.acc_end);
+    L.bytes = c.bytes() + 8192 * sizeof(double) + 512;
+    L.box = take(18 * ts + 8);
+    L.ticket = take(sizeof(unsigned));
+    L.energy = take(sizeof(double));
+    L.partials = take(8064 * sizeof(double));  // with room to align the caller's pointer
+    return L;
+  }
   L.acc = take((size_t)natoms * 4 * 8);
   L.acc_lj = take((size_t)natoms * 2 * 8);
-  L.gs_tab = take((size_t)(ntypes * ntypes) * 8);
-  L.ge_tab = take((size_t)(ntypes * ntypes) * 8);
-  L.atoms = take((size_t)natoms * 32);  // FP64 (x, y, z, q), or FP32 with room for a second vector
+  L.gs_tab = take(tab);
+  L.ge_tab = take(tab);
+  L.atoms = L.acc_end = take((size_t)natoms * 32);  // FP64 (x, y, z, q), or FP32 with room for a second vector
   L.lj = take(dtype == TFF_F64 ? (size_t)natoms * 16 : 0);
   L.box = take(18 * ts + 8);
   L.partials = take(8 * 1024 * sizeof(double));
@@ -512,7 +538,8 @@ int launch_pairs(PairArgs<T> a, int64_t total, cudaStream_t s) {
   const int nb = grid_blocks(total);
   const int64_t share = (total + (int64_t)nb * kPairBlock - 1) / ((int64_t)nb * kPairBlock);
   a.iters = (int)std::max<int64_t>(1, std::min<int64_t>(kMaxPairIters, share));
-  return launch_k(true, pair_kernel<T, CM, LM, ERF>, nb, kPairBlock, 0, s, a);
+  const auto kernel = a.atoms ? pair_kernel<T, CM, LM, ERF, true> : pair_kernel<T, CM, LM, ERF, false>;
+  return launch_k(true, kernel, nb, kPairBlock, 0, s, a);
 }
 
 template <class T>
@@ -555,16 +582,18 @@ struct PairCall {
 template <class T>
 int run_pairs(const PairCall &c, cudaStream_t s) {
   using S = typename Acc<T>::S;
-  PairLayout L = pair_layout(c.dtype, c.natoms, c.ntypes);
+  PairLayout L = pair_layout(c.dtype, c.natoms, c.ntypes, true);
+  const bool records = c.ws_bytes >= L.bytes;
+  if (!records) L = pair_layout(c.dtype, c.natoms, c.ntypes, false);
   if (c.ws_bytes < L.bytes || c.ws == nullptr) {
     set_error("workspace too small: need %zu bytes, got %zu", L.bytes, c.ws_bytes);
     return TFF_ERR_WORKSPACE;
   }
   char *ws = reinterpret_cast<char *>((reinterpret_cast<uintptr_t>(c.ws) + kWsAlign - 1) & ~uintptr_t(kWsAlign - 1));
   PairArgs<T> a{};
-  auto *atoms = reinterpret_cast<typename V4<T>::type *>(ws + L.atoms);
+  auto *atoms = records ? reinterpret_cast<typename V4<T>::type *>(ws + L.atoms) : nullptr;
   const bool wide = sizeof(T) == 4 && c.lm == L_ATOM;
-  auto *lj = c.lm == L_ATOM && !wide ? reinterpret_cast<typename LjRec<T>::type *>(ws + L.lj) : nullptr;
+  auto *lj = records && c.lm == L_ATOM && !wide ? reinterpret_cast<typename LjRec<T>::type *>(ws + L.lj) : nullptr;
   auto *box = reinterpret_cast<PairBox<T> *>(ws + L.box);
   a.atoms = atoms;
   a.lj = lj;
@@ -573,6 +602,9 @@ int run_pairs(const PairCall &c, cudaStream_t s) {
   a.npairs = c.npairs;
   a.excl = c.excl;
   a.nexcl = c.nexcl;
+  a.x = static_cast<const T *>(c.x);
+  a.q = c.cm != C_NONE ? static_cast<const T *>(c.q) : nullptr;
+  a.types = c.lm == L_TYPE ? c.types : nullptr;
   a.sig = static_cast<const T *>(c.sig);
   a.eps = static_cast<const T *>(c.eps);
   a.ntypes = c.ntypes;
@@ -597,15 +629,14 @@ int run_pairs(const PairCall &c, cudaStream_t s) {
   a.ticket = reinterpret_cast<unsigned *>(ws + L.ticket);
   a.energy = reinterpret_cast<double *>(ws + L.energy);
   // the accumulator region is cleared as far as this call uses it
-  const size_t zero = a.acc_lj || a.gs || a.ge ? L.atoms : a.acc ? L.acc_lj : 0;
+  const size_t zero = a.acc_lj || a.gs || a.ge ? L.acc_end : a.acc ? L.acc_lj : 0;
   const int64_t nacc2 = (int64_t)(zero / sizeof(ulonglong2));
   const auto blocks = [](int64_t work) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((work + kPairBlock - 1) / kPairBlock, (int64_t)sm_count() * 8));
   };
-  int st = launch_k(false, pair_prep_kernel<T>, blocks(std::max(c.natoms, nacc2)), kPairBlock, 0, s, c.natoms,
-                    static_cast<const T *>(c.x), c.cm != C_NONE ? static_cast<const T *>(c.q) : nullptr,
-                    c.lm == L_TYPE ? c.types : nullptr, a.sig, a.eps, static_cast<const T *>(c.box), atoms, wide, lj, box,
-                    reinterpret_cast<ulonglong2 *>(ws), nacc2, a.ticket);
+  int st = launch_k(false, pair_prep_kernel<T>, blocks(std::max(c.natoms, nacc2)), kPairBlock, 0, s,
+                    records ? c.natoms : (int64_t)0, a.x, a.q, a.types, a.sig, a.eps, static_cast<const T *>(c.box),
+                    atoms, wide, lj, box, reinterpret_cast<ulonglong2 *>(ws), nacc2, a.ticket);
   if (st != TFF_OK) return st;
   const int64_t total = c.npairs + (c.cm == C_EWALD ? c.nexcl : 0);
   if ((st = dispatch_pairs<T>(c.cm, c.lm, a, total, s)) != TFF_OK) return st;
@@ -733,7 +764,7 @@ int tff_nonbonded_atom_pairs_noalloc(int dtype, int64_t natoms, const void *coor
   TFF_ARG(natoms >= 0 && natoms <= kNoAllocMaxAtoms,
           "natoms=%lld exceeds the static scratch limit of %lld atoms of tff_nonbonded_atom_pairs_noalloc",
           (long long)natoms, (long long)kNoAllocMaxAtoms);
-  const size_t need = pair_layout(dtype, natoms, 0).bytes;
+  const size_t need = pair_layout(dtype, natoms, 0, true).bytes;
   TFF_ARG(need <= kNoAllocScratchBytes, "static scratch too small (%zu > %zu bytes)", need, kNoAllocScratchBytes);
   void *ws = nullptr;
   int st = noalloc_scratch(&ws);
@@ -752,7 +783,7 @@ int tff_nonbonded_atom_pairs_noalloc(int dtype, int64_t natoms, const void *coor
 }
 
 size_t tff_pairs_workspace_bytes(int dtype, int64_t natoms, int64_t ntypes) {
-  return pair_layout(dtype, natoms, ntypes).bytes;
+  return pair_layout(dtype, natoms, ntypes, true).bytes;
 }
 
 int tff_nonbonded_atom_pairs(int dtype, int64_t natoms, const void *coords, int64_t npairs,
