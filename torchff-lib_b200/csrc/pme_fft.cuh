@@ -9,8 +9,8 @@
 // A line of K = R1 R2 points is transformed in two steps (Cooley-Tukey): R2 transforms of R1
 // points with stride R2, a twiddle, R1 transforms of R2 consecutive points. A step's transforms
 // are unrolled in one thread's registers (radix up to kMaxRegRadix, again by Cooley-Tukey with
-// constant twiddles; odd primes by sums over a[j] + a[R-j] and a[j] - a[R-j]); a larger prime
-// factor of K is a direct sum from shared memory. Two real lines go through the z transform as
+// constant twiddles; odd primes by sums over a[j] + a[R-j] and a[j] - a[R-j]); for a larger prime
+// factor of K those sums run from shared memory. Two real lines go through the z transform as
 // one complex line. Lanes take consecutive lines: on an odd row pitch they hit distinct banks, and
 // the twiddles they share are broadcasts. Summation orders are fixed.
 //
@@ -63,11 +63,12 @@ inline size_t fft_smem(int K) {
 }
 
 // Grid sides of the plane path: up to 78, both buffers of an FP64 plane fit the shared memory of a
-// block. Sides with a factor beyond the registers only up to 36: their direct sums grow as K^2
-// a line. One energy with gradients of 3,000 charges, cuFFT -> planes, us, FP32: K = 16 37.5 -> 26.1,
-// 34 51.3 -> 39.2, 37 39.9 -> 42.8, 48 40.1 -> 32.9, 67 56 -> 110, 78 55.1 -> 52.4, 80 46.1 -> 53.1,
-// 100 53.7 -> 64.4; FP64: 34 53.2 -> 41.2, 37 41.3 -> 46.6, 48 40.3 -> 34.4, 78 85.4 -> 56.4, 80 52.8 ->
-// 55.7.
+// block. One energy with gradients of 3,000 charges, cuFFT -> planes, us, FP32: K = 16 37.5 -> 26.1,
+// 34 51.3 -> 36.9, 48 40.1 -> 32.9, 78 55.1 -> 52.4, 80 46.1 -> 53.1, 100 53.7 -> 64.4; FP64: 34 53.2 -> 38.8,
+// 48 40.3 -> 34.4, 78 85.4 -> 56.4, 80 52.8 -> 55.7. Sides with a factor beyond the registers only up to 36:
+// the sums of a factor R grow as R^2. Prime sides tie to 53 (FP32 energies alone: 41 39.0 -> 37.0, 47 39.1 -> 41.3,
+// 53 45.2 -> 45.2) and lose beyond (59 47.2 -> 54.9, 67 53.4 -> 65.7); twice or three times a prime can still win
+// (46 51.3 -> 41.2, 51 61.5 -> 41.0, 58 55.6 -> 50.2), four times does not (68 43.1 -> 53.3, 76 47.4 -> 65.3).
 inline bool fft_planes(int K) { return K <= 78 && (K <= 36 || K / fft_radix1(K) <= kMaxRegRadix); }
 
 // Layout of a block's shared memory, in elements: plane p with the data, the other plane q, the table.
@@ -109,12 +110,6 @@ template <class T, bool INV>
 __device__ __forceinline__ Cplx<T> cmul(Cplx<T> a, Cplx<T> w) {
   const T wy = INV ? -w.y : w.y;
   return Cplx<T>{fma(a.x, w.x, -a.y * wy), fma(a.x, wy, a.y * w.x)};
-}
-template <class T, bool INV>
-__device__ __forceinline__ void cmac(Cplx<T> &s, Cplx<T> a, Cplx<T> w) {
-  const T wy = INV ? -w.y : w.y;
-  s.x = fma(-a.y, wy, fma(a.x, w.x, s.x));
-  s.y = fma(a.y, w.x, fma(a.x, wy, s.y));
 }
 
 // cos(2 pi k / n) as a constant: the angle is folded into [0, pi / 4] in whole numbers, then the
@@ -219,10 +214,10 @@ __device__ __forceinline__ void reg_dft(Cplx<T> (&a)[R]) {
 
 // One step over `lines` lines (element n of line l at l * pitch_line + n * pitch_el): transforms of R
 // points, `groups` per line. Group g reads elements g * in_g + n * in_s and writes elements
-// g * out_g + k * out_s below `kmax`; with `twiddle` output k of group g is multiplied by tw[g k].
+// g * out_g + k * out_s; with `twiddle` output k of group g is multiplied by tw[g k].
 struct FftStep {
   int R, groups, lines, pitch_line, pitch_el;
-  int in_g, in_s, out_g, out_s, kmax;
+  int in_g, in_s, out_g, out_s;
   int in, out;  // plane read, plane written
   bool twiddle;
 };
@@ -244,39 +239,75 @@ __device__ __forceinline__ void fft_step_r(const FftStep &s, int tw) {
       for (int k = 0; k < R; ++k) dst[k * os] = k ? cmul<T, INV>(a[k], *fft_at<T>(tw + g * k)) : a[k];
     } else {
 #pragma unroll
-      for (int k = 0; k < R; ++k)
-        if (g * s.out_g + k * s.out_s < s.kmax) dst[k * os] = a[k];
+      for (int k = 0; k < R; ++k) dst[k * os] = a[k];
     }
   }
 }
 
-// Any radix: four outputs at a time, inputs read once per four.
+// The last step of a line whose radix does not fit the registers, an odd one: outputs k and R - k of
+// kAnyPairs values of k at a time from the sums and differences of inputs j and R - j (as in
+// reg_dft): half the multiply-adds of a direct sum, and the inputs read once for all of them. By count it
+// is bound by shared memory, four loads for eight multiply-adds. An evaluation of a batch of 16 boxes of
+// 300 to 1,050 waters, FP32, us, against four outputs of a direct sum per thread: K = 37 284 -> 251,
+// 47 380 -> 296, 71 1,129 -> 693, 89 2,272 -> 1,169; a lone 3,000-charge grid at K = 31 40.6 -> 34.9. Two values
+// of k leave the fewest threads without work at small K; three or four change K = 53 to 94 by -6 to +7 %.
+constexpr int kAnyPairs = 2;
+
+constexpr bool any_radix_is_odd() {
+  for (int K = 6; K <= 96; ++K) {
+    int r = 1;
+    for (int d = 2; d * d <= K; ++d)
+      if (K % d == 0) r = d;
+    if (r > kMaxRegRadix || (K / r > kMaxRegRadix && K / r % 2 == 0)) return false;
+  }
+  return true;
+}
+static_assert(any_radix_is_odd(), "grid sides up to 96: a radix beyond the registers is odd and the last step's");
+
 template <class T, bool INV>
 __device__ __forceinline__ void fft_step_any(const FftStep &s, int tw, int stride) {
-  const int R = s.R, blocks = (R + 3) / 4;
+  const int R = s.R, H = (R - 1) / 2, blocks = (H + kAnyPairs - 1) / kAnyPairs;
   const SmallDiv by(s.lines), byb(blocks);
+  const int is = s.in_s * s.pitch_el, os = s.out_s * s.pitch_el;
   for (int t = threadIdx.x; t < s.lines * s.groups * blocks; t += blockDim.x) {
-    const int gb = by.quot(t), l = t - gb * s.lines, g = byb.quot(gb), k0 = 4 * (gb - g * blocks);
-    if (g * s.out_g + k0 * s.out_s >= s.kmax) continue;
+    const int gb = by.quot(t), l = t - gb * s.lines, g = byb.quot(gb), k0 = 1 + kAnyPairs * (gb - g * blocks);
     const Cplx<T> *src = fft_at<T>(s.in + l * s.pitch_line + g * s.in_g * s.pitch_el);
     Cplx<T> *dst = fft_at<T>(s.out + l * s.pitch_line + g * s.out_g * s.pitch_el);
-    Cplx<T> v[4] = {};
-    int m[4] = {};
-#pragma unroll 4
-    for (int n = 0; n < R; ++n) {
-      const Cplx<T> a = src[n * s.in_s * s.pitch_el];
+    const Cplx<T> a0 = src[0];
+    Cplx<T> sum = a0, u[kAnyPairs], v[kAnyPairs];
+    int m[kAnyPairs];  // j k mod R
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        cmac<T, INV>(v[u], a, *fft_at<T>(tw + m[u] * stride));
-        m[u] += k0 + u < R ? k0 + u : 0;  // n k mod R
-        m[u] -= m[u] >= R ? R : 0;
+    for (int q = 0; q < kAnyPairs; ++q) {
+      u[q] = a0;
+      v[q] = Cplx<T>{T(0), T(0)};
+      m[q] = 0;
+    }
+#pragma unroll 4
+    for (int j = 1; j <= H; ++j) {
+      const Cplx<T> a = src[j * is], b = src[(R - j) * is];
+      const Cplx<T> p{a.x + b.x, a.y + b.y}, d{a.x - b.x, a.y - b.y};
+      sum.x += p.x;
+      sum.y += p.y;
+#pragma unroll
+      for (int q = 0; q < kAnyPairs; ++q) {
+        m[q] += k0 + q;
+        m[q] -= m[q] >= R ? R : 0;
+        const Cplx<T> w = *fft_at<T>(tw + m[q] * stride);
+        const T n = INV ? w.y : -w.y;
+        u[q].x = fma(w.x, p.x, u[q].x);
+        u[q].y = fma(w.x, p.y, u[q].y);
+        v[q].x = fma(n, d.x, v[q].x);
+        v[q].y = fma(n, d.y, v[q].y);
       }
     }
+    if (k0 == 1) dst[0] = sum;
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int k = k0 + u;
-      if (k >= R || g * s.out_g + k * s.out_s >= s.kmax) continue;
-      dst[k * s.out_s * s.pitch_el] = s.twiddle ? cmul<T, INV>(v[u], *fft_at<T>(tw + g * k)) : v[u];
+    for (int q = 0; q < kAnyPairs; ++q) {
+      const int k = k0 + q;
+      if (k > H) continue;
+      // u - i v and its mirror u + i v
+      dst[k * os] = Cplx<T>{u[q].x + v[q].y, u[q].y - v[q].x};
+      dst[(R - k) * os] = Cplx<T>{u[q].x - v[q].y, u[q].y + v[q].x};
     }
   }
 }
@@ -306,10 +337,10 @@ __device__ __noinline__ void fft_step(const FftStep s, int tw, int K) {
   }
 }
 
-// Transforms `lines` lines of plane f.p; outputs below `kmax` only. The result is in f.p again (the
-// planes swap when K is prime). All threads of the block; ends with the result visible to it.
+// Transforms `lines` lines of plane f.p. The result is in f.p again (the planes swap when K is
+// prime). All threads of the block; ends with the result visible to it.
 template <class T, bool INV>
-__device__ __forceinline__ void fft_lines(FftPlan &f, int lines, int pitch_line, int pitch_el, int kmax) {
+__device__ __forceinline__ void fft_lines(FftPlan &f, int lines, int pitch_line, int pitch_el) {
   FftStep s;
   s.lines = lines;
   s.pitch_line = pitch_line;
@@ -319,7 +350,6 @@ __device__ __forceinline__ void fft_lines(FftPlan &f, int lines, int pitch_line,
     s.R = f.R1;
     s.groups = s.in_s = s.out_s = f.R2;
     s.in_g = s.out_g = 1;
-    s.kmax = f.K;
     s.out = f.q;
     s.twiddle = true;
     fft_step<T, INV>(s, f.tw, f.K);
@@ -329,7 +359,6 @@ __device__ __forceinline__ void fft_lines(FftPlan &f, int lines, int pitch_line,
   s.R = s.in_g = f.R2;
   s.groups = s.out_s = f.R1;
   s.in_s = s.out_g = 1;
-  s.kmax = kmax;
   s.out = f.R1 > 1 ? f.p : f.q;
   s.twiddle = false;
   fft_step<T, INV>(s, f.tw, f.K);
@@ -358,7 +387,7 @@ __device__ __forceinline__ void fft_forward_plane(FftPlan &f, const typename Acc
                                            2 * m + 1 < K ? fft_real(grid[(2 * m + 1) * K + z]) : T(0)};
   }
   __syncthreads();
-  fft_lines<T, false>(f, pairs, st, 1, K);
+  fft_lines<T, false>(f, pairs, st, 1);
   // their spectra: (Z[k] + conj Z[-k]) / 2 and (Z[k] - conj Z[-k]) / 2i
   for (int t = threadIdx.x; t < pairs * Kz; t += blockDim.x) {
     const int m = byz.quot(t), z = t - m * Kz;
@@ -370,7 +399,7 @@ __device__ __forceinline__ void fft_forward_plane(FftPlan &f, const typename Acc
   f.q = f.p;
   f.p = spec;
   __syncthreads();
-  fft_lines<T, false>(f, Kz, 1, st, K);
+  fft_lines<T, false>(f, Kz, 1, st);
   before_store();
   for (int t = threadIdx.x; t < K * Kz; t += blockDim.x) {
     const int y = byz.quot(t);
@@ -389,10 +418,12 @@ __device__ __forceinline__ void fft_inverse_plane(FftPlan &f, const Cplx<T> *in,
     *fft_at<T>(f.p + y * st + t - y * Kz) = in[t];
   }
   __syncthreads();
-  fft_lines<T, true>(f, Kz, 1, st, K);
+  fft_lines<T, true>(f, Kz, 1, st);
   // line m = A + i B of the half spectra A, B of rows 2m and 2m + 1: its transform has their real
   // lines as real and imaginary parts. The other half is conj A[K - k] + i conj B[K - k]. The
-  // imaginary parts of k = 0 and K / 2, zero but for rounding, have no real counterpart.
+  // imaginary parts of k = 0 and K / 2 have no real counterpart: they are dropped, as in
+  // cuFFT's C2R. They vanish but for rounding where the influence function of a frequency and of its mirror
+  // image are equal, which the Nyquist frequencies of an even K in a sheared box are not.
   for (int t = threadIdx.x; t < pairs * Kz; t += blockDim.x) {
     const int m = byz.quot(t), z = t - m * Kz;
     const bool own = z == 0 || 2 * z == K;
@@ -406,7 +437,7 @@ __device__ __forceinline__ void fft_inverse_plane(FftPlan &f, const Cplx<T> *in,
   f.q = f.p;
   f.p = lines;
   __syncthreads();
-  fft_lines<T, true>(f, pairs, st, 1, K);
+  fft_lines<T, true>(f, pairs, st, 1);
   before_store();
   for (int t = threadIdx.x; t < pairs * K; t += blockDim.x) {
     const int m = byk.quot(t), z = t - m * K;
@@ -442,7 +473,7 @@ __device__ __forceinline__ double fft_solve_row(FftPlan &f, Cplx<T> *spec, int k
     *fft_at<T>(f.p + x * st + z) = spec[((size_t)x * K + ky) * Kz + z0 + z];
   }
   __syncthreads();
-  fft_lines<T, false>(f, nz, 1, st, K);
+  fft_lines<T, false>(f, nz, 1, st);
   double e = 0.0;
   const auto apply = [&](int t, double c) {
     const int x = byn.quot(t), z = t - x * nz;
@@ -462,7 +493,7 @@ __device__ __forceinline__ double fft_solve_row(FftPlan &f, Cplx<T> *spec, int k
     apply(t, factor(x, z0 + t - x * nz));
   }
   __syncthreads();
-  fft_lines<T, true>(f, nz, 1, st, K);
+  fft_lines<T, true>(f, nz, 1, st);
   before_store();
   for (int t = threadIdx.x; t < total; t += blockDim.x) {
     const int x = byn.quot(t), z = t - x * nz;
