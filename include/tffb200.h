@@ -294,7 +294,9 @@ int tff_angles(int dtype, int64_t natoms, const void *coords, int64_t nangles,
 
 typedef struct tff_pme_plan_s *tff_pme_plan;
 
-/* Creates the cuFFT R2C/C2R plans (cuFFT allocates its own work area here). */
+/* Creates the transform tables, or the cuFFT R2C/C2R plans (cuFFT allocates its own work area here)
+ * of grid sides that the library's own plane transforms do not take: above 78, and above 36 when the
+ * larger of the two factors K = R1 R2 closest to each other exceeds 16 (37, 46, 51, ...). */
 int tff_pme_plan_create(int dtype, int K, tff_pme_plan *plan);
 int tff_pme_plan_destroy(tff_pme_plan plan);
 size_t tff_pme_workspace_bytes(tff_pme_plan plan, int64_t natoms);
@@ -414,8 +416,9 @@ int tff_system_kernel_launches(tff_system sys);
  * precision: bit-identical whatever else is in the batch). Same physics as tff_system_*;
  * cutoff, Ewald alpha and the Coulomb constant are shared by the batch.
  * Per system: 1 <= natoms <= 16384, 6 <= K <= 96 (TFF_F32) or 64 (TFF_F64). The
- * reciprocal-space transforms take all grid sizes in the same three launches, with the
- * arithmetic of a single system's.
+ * reciprocal-space transforms take all grid sizes in the same three launches. For the grid
+ * sides that single systems do not leave to cuFFT (see tff_pme_plan_create) the arithmetic is that
+ * of a single system; the others match it to FP rounding.
  * --------------------------------------------------------------------------- */
 typedef struct tff_batch_s *tff_batch;
 

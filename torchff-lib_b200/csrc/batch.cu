@@ -236,7 +236,6 @@ int batch_prepare(tff_batch b, int nsys, const int64_t *natoms, const int *pme_g
   sh.total_grid = go;
   sh.nsys = nsys;
   sh.plane_units = planes;
-  sh.kmax = kmax;
   sh.gather_units = gat;
   // the pinned block is reused once the previous upload out of it is done
   TFF_CUDA(cudaEventSynchronize(b->table_ev));

@@ -168,7 +168,6 @@ struct BatchShape {
   int64_t natoms, nclusters, npad, nsuper, total_grid;
   int nsys;
   int plane_units;  // transform planes: sum of K
-  int kmax;
   int gather_units; // gather (and spread) units: sum of gather_blocks
   int pad;
 };
@@ -855,9 +854,13 @@ __global__ void slot_params_kernel(ClusterData<T> d, SlotParams<T> params) {
 
 // While the blocks of the neighbour search leave SMs idle (up to 592 clusters), more blocks of that
 // launch write the slot parameters, and the real-space kernels find an item's cluster by item_cluster:
-// one launch less, 3,000 waters 81.9 -> 79.1 us, FP64 144 -> 140 us, 1,231 flexible waters 77 -> 73 us. With
-// more clusters a launch of its own follows, which also writes the cluster of each item: the same
-// at every size took 300,000 atoms from 1,231 to 1,270 us and a batch of 60 boxes from 724 to 767 us.
+// one launch less, 3,000 waters 81.9 -> 79.1 us (though the search for an item's cluster makes the pair
+// kernel 1 us longer), FP64 144 -> 140 us, 1,231 flexible waters 77 -> 73 us. With more clusters a launch
+// of its own follows, which also writes the cluster of each item: the same at every size took
+// 300,000 atoms from 1,231 to 1,270 us and a batch of 60 boxes from 724 to 767 us. Between 400 and 1,000
+// clusters neither side is better throughout; beside / after, us, FP32 at 469, 563, 592, 657, 938 and 1,125
+// clusters: 101 / 98, 140 / 142, 136 / 134, 133 / 126, 172 / 177, 181 / 175; FP64 at 282, 469, 592, 938
+// and 1,125: 120 / 126, 170 / 174, 225 / 222, 311 / 317, 361 / 359.
 inline bool slots_beside_search(int64_t clusters) { return clusters <= 4 * (int64_t)sm_count(); }
 
 inline int slot_blocks(int64_t slots, int threads) {
@@ -1013,7 +1016,8 @@ __global__ void cluster_neighbors_kernel(ClusterData<T> d, double rc, int half, 
 // Steps 1-6 of a small system in one launch of one block: a thread per atom, a warp per cluster.
 // Up to kSmallAtoms atoms (32 clusters, one super-cluster) the six launches of the general build
 // are latency from end to end (648 atoms: 34 us of kernels, 41 with the slot parameters; this one 8.8
-// and 13.7 us); the sort order, boxes, lists and work items are the same.
+// and 13.7 us); the sort order, boxes, lists and work items are the same (super-cluster boxes, which only
+// the general search reads, are not written).
 constexpr int kSmallAtoms = 1024;
 constexpr int kSmallKeys = 512;  // the cell grid of 1024 atoms: 5 cells per side, 3 bits per axis
 
@@ -1117,7 +1121,6 @@ __global__ void __launch_bounds__(kSmallAtoms) small_build_kernel(const T *x, co
     if (lane == 0) s_h[w] = h;
   }
   __syncthreads();
-  if (w == 0) super_box(d, 0, ncl, lane, lane < ncl ? s_c[lane] : V{}, lane < ncl ? s_h[lane] : V{}, s_c[0]);
   // neighbour lists: lane J against cluster w
   int count = 0;
   if (w < ncl) {

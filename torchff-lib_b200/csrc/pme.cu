@@ -15,7 +15,9 @@ int pme_cufft_fail(cufftResult r, const char *what) {
 namespace {
 
 // The three launches of a solve over planes (pme_fft.cuh), programmatic dependents of the kernel
-// before: a kernel copies its tables (and works out its influence function) while that one ends.
+// before: a kernel copies its tables (and works out its influence function) while that one ends; no
+// kernel of the chain writes tables, box or moduli, and the forward kernel lets the solve start only after
+// its own wait, so whatever wrote the box has completed by then (the rule of launch_k).
 // A block lets the next kernel start only when it has nothing but its result left to write, so
 // that waiting blocks do not sit on SMs that the real-space stream could use. The solve's blocks
 // split a row's kz range so that small grids use every SM.

@@ -59,7 +59,11 @@ __device__ __forceinline__ void pdl_enter() {
 }
 
 // Launches `kernel` on `s`; with `pdl` as a programmatic dependent of the previous kernel in
-// the stream (the kernel must begin with pdl_enter()).
+// the stream. Such a kernel waits (griddepcontrol.wait) before it touches anything that an unfinished
+// kernel may write, and lets its own dependents start (griddepcontrol.launch_dependents, or its end)
+// only after that wait. When a kernel of a chain starts, every kernel but the one before it has
+// then completed, so before its wait it may read what older ones wrote. pdl_enter() as the first statement does
+// both; the plane transforms of the PME solve (pme.cu) read their tables and the box before the wait.
 template <class... P, class... A>
 int launch_k(bool pdl, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A &&...args) {
   cudaLaunchConfig_t cfg = {};

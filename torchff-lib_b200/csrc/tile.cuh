@@ -169,7 +169,6 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? kTileMi
       x_lo = __reduce_min_sync(kFull, lo);
       x_hi = __reduce_max_sync(kFull, hi);
     }
-    bool all_shifted = true;  // warp-uniform: no tile of the item needs the per-pair minimum image
 
     // stage the tiles and build their cutoff masks (pass 1)
     for (int t = 0; t < ntile; ++t) {
@@ -285,7 +284,6 @@ __global__ void __launch_bounds__(TileCfg<T, MODE>::NW * 32, MODE == 0 ? kTileMi
       s_mask[w][t][lane] = mask & ~emask;
       s_xmask[w][t][lane] = mask & emask;
       if (lane == 0) s_mi[w][t] = !shifted;
-      all_shifted = all_shifted && shifted;
     }
     __syncwarp();
 
