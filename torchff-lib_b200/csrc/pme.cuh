@@ -271,9 +271,8 @@ struct IndexedGatherOut {
 // -(a/sqrt(pi)) sum q^2.
 //
 // The lanes are those of the spread: six along z and five (x, y) rows at a time, so that a load
-// touches runs of six consecutive points (an x plane per lane touched 30 rows with every load,
-// and the L1 lookups bound the kernel: 95 % of its throughput). A lane sums its rows against the
-// x and y weights, then multiplies by its z weights; the four sums of four atoms are
+// touches runs of six consecutive points (an x plane per lane touched 30 rows with every load). A lane
+// sums its rows against the x and y weights, then multiplies by its z weights; the four sums of four atoms are
 // reduce-scattered over the warp together, one shuffle per value instead of five. 9,000 atoms FP32
 // 11.9 -> 9.9 us; an energy with gradients of 30,000 scattered charges in FP64 121 -> 112 us.
 constexpr int kGatherAtoms = 4;

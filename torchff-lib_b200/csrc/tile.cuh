@@ -76,7 +76,7 @@ __device__ __forceinline__ void pair_min_image(bool ortho, T &dx, T &dy, T &dz, 
 }
 
 // Resident 2-warp blocks per SM the register allocation of the FP64 energy kernel must allow: 10 (at
-// most 96 registers). 3000 waters: 141 us per evaluation, 147 at 6 (104 registers), 150 at 13 (72).
+// most 96 registers). 3000 waters: 141 us per evaluation, 148 at 6, 149 at 13 (72 registers).
 constexpr int kTileMinBlocks = 10;
 
 // ERF (FP64): how the screened Coulomb terms are evaluated (erf_poly.cuh).
